@@ -874,6 +874,18 @@ void keep_pool_memory(int dev) {
     done.push_back(dev);
 }
 
+// Planes per z-chunk of a sweep with `bp` block-planes (blocks of one plane, times planes), for
+// 2 x 148 resident blocks.  A chunk costs its planes and about 0.4 of a plane more (its first plane
+// waits for memory with nothing to overlap), and the last blocks of a launch run alone for about
+// 0.9 of a chunk: bp / 296 (1 + 0.4 / c) + 0.9 c, least at c = sqrt(0.46 bp / 296).  Fitted to FP32
+// and FP64 solves from 48^3 to 400^3 swept over c = 1, 2, 3, 4, 6, 10, 16; the fastest of these is
+// the rule's or a neighbour within 2 %.  Before, a chunk had 8 planes or more, which on a small
+// grid is that many memory latencies in a row on a few blocks: us per step with chunks of 8 -> now,
+// 48^3 FP32 (c = 1) 48 -> 20, 80^3 (1) 53 -> 27, 201x201x69 (2) 93 -> 88, 173x131x97 FP64 (3)
+// 115 -> 109.  Above 16 planes the blocks' unequal work (edge columns, CPML rows) costs more than
+// longer chunks save (536^3: 16 planes 1.107 ms, 34 planes 1.159 ms for the FP32 E sweep).
+int sweep_chunk(double bp) { return int(std::clamp(std::lround(std::sqrt(0.46 * bp / 296.0)), 1l, 16l)); }
+
 // The setup's full-grid checks that need no device: the material index's range and the gain
 // cells' bounding box and placement.  A large solve runs them on a helper thread while it
 // allocates its device arrays (for a 536^3 first solve both take tens of milliseconds: growing
@@ -1264,20 +1276,9 @@ Solver<S, T>::Solver(const fdtd_setup_v1& s, int dev, const ShardSpec* shard, bo
     g.er = g.ne ? (32 * kBlockY) / g.ne : 1;
     const int gxH = g.gxi + (g.ne ? 1 : 0), gxE = gxi_E<S>(g) + (g.ne ? 1 : 0);
     const int gyE = std::max((NyT_ + rows_blk - 1) / rows_blk, g.ne ? (NyT_ + g.er - 1) / g.er : 0);
-    // launch shapes: z-chunks of at most 16 planes, and enough of them that the grid holds
-    // several waves of blocks.  Measured on the 536^3 CPML + gain workload (one B200): chunks
-    // of 67 -> 34 -> 16 planes take the E sweep from 1.258 to 1.159 to 1.107 ms (FP32) and from
-    // 1.006 to 0.900 to 0.868 ms (BF16), the H sweep from 1.025 to 0.972 ms (FP32); 12 and 8
-    // planes are no faster.  Short chunks balance the blocks' work (a chunk of an edge column
-    // or a CPML row runs longer than an interior one) and shorten the last wave.
-    auto chunk = [&](int rows, int planes, int gx) {
-        const int bxy = std::max(1, gx * ((rows + rows_blk - 1) / rows_blk));
-        const int want = std::max(1, (148 * 16 + bxy - 1) / bxy);
-        const int zc = std::max({1, std::min(want, std::max(1, planes / 8)), (planes + 15) / 16});
-        return std::max(1, (planes + zc - 1) / zc);
-    };
-    kchunkH_ = chunk(NyT_ - 1, NzT_ - 1, gxH);
-    kchunkE_ = chunk(NyT_, NzT_, gxE);
+    // launch shapes: z-chunks by the rule of sweep_chunk
+    kchunkH_ = sweep_chunk(double(gxH) * ((NyT_ - 1 + rows_blk - 1) / rows_blk) * (NzT_ - 1));
+    kchunkE_ = sweep_chunk(double(gxE) * ((NyT_ + rows_blk - 1) / rows_blk) * NzT_);
     if (const char* e = std::getenv("FDTD_B200_KCHUNK")) kchunkH_ = kchunkE_ = std::max(1, std::atoi(e));
     if (gyE > 65535) throw Failure(FDTD_ERR_INVALID, "grid too large for the sweep launch shape (NyT)");
     gridH_ = dim3(gxH, gyE, std::max(1, (a.kH1 + kchunkH_ - 1) / kchunkH_));
@@ -2304,6 +2305,15 @@ private:
         std::vector<BatchSolve> bs(n);
         std::vector<int4> tab;
         std::vector<int> ekind(n), form(n);
+        // z-chunks for the whole launch: the resident solves share the GPU, so the block-planes
+        // of all of them decide, not those of each
+        double bpH = 0, bpE = 0;
+        for (int r = 0; r < n; ++r)
+            with(jobs_.at(res_[r]), [&](auto& v) {
+                bpH += double(v.gridH_.x) * v.gridH_.y * v.NzT_;
+                bpE += double(v.gridE_.x) * v.gridE_.y * v.NzT_;
+            });
+        const int kcH = sweep_chunk(bpH), kcE = sweep_chunk(bpE);
         for (int r = 0; r < n; ++r) {
             Job& j = jobs_.at(res_[r]);
             BatchSolve& b = bs[r];
@@ -2313,8 +2323,8 @@ private:
             else args[r].bf16 = j.bf16->a_;
             with(j, [&](auto& v) {
                 b.g = v.geom_;
-                b.kchunkH = kchunk_ ? kchunk_ : v.kchunkH_;
-                b.kchunkE = kchunk_ ? kchunk_ : v.kchunkE_;
+                b.kchunkH = kchunk_ ? kchunk_ : kcH;
+                b.kchunkE = kchunk_ ? kchunk_ : kcE;
                 b.probes = v.d_probes_;
                 b.nprobes = int(v.nprobes_);
                 b.nf = int(v.nf_);
@@ -2529,12 +2539,9 @@ private:
     int poll_n_ = 0;
     unsigned* h_status_ = nullptr;
     // Launch shape: staged sweeps (the E sweep for every storage form, the H sweep for 16-bit
-    // storage, as for a single solve: staging the FP32 H sweep costs 4 %) and each solve's own
-    // z-chunks (at most 16 planes, shorter on small grids so that a lone solve still fills the
-    // GPU; 16-plane chunks for every solve had measured 1.19 -> 1.12 ms per packed step of 64
-    // BF16 cavities of 96x96x64 against each solve's chunks of the time, which were up to 64
-    // planes).  FDTD_B200_BATCH_KCHUNK (planes, 0 = each solve's own) / _H_PIPE / _E_PIPE
-    // override them.
+    // storage, as for a single solve: staging the FP32 H sweep costs 4 %) and the z-chunks of
+    // sweep_chunk for all resident solves' blocks together (rebuild).  FDTD_B200_BATCH_KCHUNK
+    // (planes, 0 = that rule) / _H_PIPE / _E_PIPE override them.
     bool hpipe_ = true, epipe_ = true;
     int kchunk_ = 0;
     // A lone resident solve steps with the single-solve launches (FDTD_B200_BATCH_SOLO=0: packed).
