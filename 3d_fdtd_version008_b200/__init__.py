@@ -384,7 +384,7 @@ class Solver:
         return {"steps": t.steps, "run_ms": t.run_ms, "h_ms": t.h_ms, "e_ms": t.e_ms, "aux_ms": t.aux_ms}
 
     def set_kernel_path(self, path: int) -> None:
-        """1 = separate H and E sweeps (default), 2 = slab-ordered step; before the first step (0 is refused)."""
+        """1 = default (separate H and E sweeps, or one fused launch by size), 2 = slab-ordered step; before the first step (0 is refused)."""
         self._check(load_library().fdtd_set_kernel_path(self._h, int(path)), "fdtd_set_kernel_path")
 
     def synchronize(self) -> None:

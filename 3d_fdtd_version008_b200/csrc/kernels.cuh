@@ -15,8 +15,9 @@
 //                with psi_E fused (src/fdtd_stepper.hpp:49-89, src/two_level_system.hpp:299-342,
 //                src/boundary.hpp:227-300), then the population update with E^{n+1}
 //                (src/two_level_system.hpp:612-666), all in one pass over the cell.
-// CPML psi lives only in the PML slabs: x-slab [k][j][2np], y-slab [k][2np][NxP],
-// z-slab [2np][j][NxP], index 0 for the low side, np.. for the high side.
+// CPML psi lives only in the PML slabs: y-slab [k][2np][NxP], z-slab [2np][j][NxP], index 0 for
+// the low side, np.. for the high side; x-slab [k][j][xlen], the W-cell vectors that hold a
+// slab cell (those on the low side, then those on the high side; XSlab).
 #pragma once
 
 #include <cuda_bf16.h>
@@ -342,37 +343,35 @@ struct ESrc {
 __device__ __forceinline__ bool in_pml(int n, int N, int np) { return n < np || n >= N - np; }
 __device__ __forceinline__ int slab_index(int n, int N, int np) { return n < np ? n : n - (N - 2 * np); }
 
-// x-slab psi ([k][j][2 np]) of one W-cell vector.  Both arrays are read before any psi
+// x-slab psi of the W-cell vector at i0 (one that holds a slab cell).  Both arrays are read before any psi
 // store is issued: the compiler may not move a load of one psi array above a store to the
 // other, and a read-after-store chain per cell would cost one memory round trip each.
+struct XSlab {
+    int lo, hi, len;  // vectors on the low side, first vector on the high side, cells of a psi row
+    __host__ __device__ __forceinline__ XSlab(int NxT, int np, int W)
+        : lo((np + W - 1) / W), hi((NxT - np) / W), len((lo + (NxT + W - 1) / W - hi) * W) {}
+};
+template <typename S, typename T>
+__device__ __forceinline__ size_t xpsi_at(const StepArgs<S, T>& a, int k, int j, int i0) {
+    const XSlab x(a.NxT, a.np, Vec<T>::W);
+    const int v = i0 / Vec<T>::W;
+    return (size_t(k) * a.NyT + j) * x.len + size_t(v < x.lo ? v : v - x.hi + x.lo) * Vec<T>::W;
+}
 template <typename S, typename T>
 __device__ __forceinline__ void xpsi_load(const S* p3, const S* p4, const StepArgs<S, T>& a, int k, int j, int i0,
                                           T (&x3)[Vec<T>::W], T (&x4)[Vec<T>::W]) {
-    const size_t row = (size_t(k) * a.NyT + j) * (2 * a.np);
-#pragma unroll
-    for (int e = 0; e < Vec<T>::W; ++e) {
-        const int i = i0 + e;
-        const bool in = i < a.NxT && in_pml(i, a.NxT, a.np);
-        const size_t q = row + (in ? slab_index(i, a.NxT, a.np) : 0);
-        x3[e] = in ? T(to_c(p3[q])) : T(0);
-        x4[e] = in ? T(to_c(p4[q])) : T(0);
-    }
+    const size_t q = xpsi_at(a, k, j, i0);
+    Fld<S, T>::ld(p3 + q, x3);
+    Fld<S, T>::ld(p4 + q, x4);
 }
 
-// Writes back the x-slab psi of the cells ilo <= i < ihi of the vector.
+// Writes back the vector's x-slab psi (cells outside the slab keep what was loaded).
 template <typename S, typename T>
-__device__ __forceinline__ void xpsi_store(S* p3, S* p4, const StepArgs<S, T>& a, int k, int j, int i0, int ilo, int ihi,
+__device__ __forceinline__ void xpsi_store(S* p3, S* p4, const StepArgs<S, T>& a, int k, int j, int i0,
                                            const T (&x3)[Vec<T>::W], const T (&x4)[Vec<T>::W]) {
-    const size_t row = (size_t(k) * a.NyT + j) * (2 * a.np);
-#pragma unroll
-    for (int e = 0; e < Vec<T>::W; ++e) {
-        const int i = i0 + e;
-        if (i >= ilo && i < ihi && in_pml(i, a.NxT, a.np)) {
-            const size_t q = row + slab_index(i, a.NxT, a.np);
-            put(p3[q], x3[e]);
-            put(p4[q], x4[e]);
-        }
-    }
+    const size_t q = xpsi_at(a, k, j, i0);
+    Fld<S, T>::st(p3 + q, x3);
+    Fld<S, T>::st(p4 + q, x4);
 }
 
 // One row (bEx, bEy, bEz) of the indexed material's table.
@@ -624,7 +623,7 @@ __device__ __forceinline__ void h_column(const StepArgs<S, T>& a, const SweepGeo
     const int jy = ypml ? slab_index(j, a.NyT, np) : 0;
     T yb = 1, yc = 0, yik = 1;
     if (ypml) { yb = __ldg(a.pbH[1] + j); yc = __ldg(a.pcH[1] + j); yik = __ldg(a.ik[1] + j); }
-    const bool xpml = EDGE && act && (i0 < np || i0 + W > a.NxT - np);
+    const bool xpml = EDGE && act && np > 0 && (i0 < np || i0 + W > a.NxT - np);
     const bool plain_row = act && !ypml && !xpml && i0 + W <= a.NxT - 1;
     // Ey, Ez at i0+W come from memory at the end of the row segment, at the end of the
     // interior (the next lane then holds no interior vector) and for every edge column
@@ -778,7 +777,7 @@ __device__ __forceinline__ void h_column(const StepArgs<S, T>& a, const SweepGeo
             st_field<SRM>(a, a.Hz, c, hz, 5, step);
             if (zpml) { Fld<S, T>::st(a.psiH[1] + zs, pxz); Fld<S, T>::st(a.psiH[2] + zs, pyz); }
             if (ypml) { Fld<S, T>::st(a.psiH[0] + ys, pxy); Fld<S, T>::st(a.psiH[5] + ys, pzy); }
-            if (xpml) xpsi_store<S, T>(a.psiH[3], a.psiH[4], a, k, j, i0, 0, a.NxT - 1, x3, x4);
+            if (xpml) xpsi_store<S, T>(a.psiH[3], a.psiH[4], a, k, j, i0, x3, x4);
         }
 #pragma unroll
         for (int e = 0; e < W; ++e) { ex0[e] = ex1[e]; ey0[e] = ey1[e]; }
@@ -1032,7 +1031,7 @@ __device__ __forceinline__ void e_column(const StepArgs<S, T>& a, const SweepGeo
     const int jy = ypml ? slab_index(j, a.NyT, np) : 0;
     T yb = 1, yc = 0, yik = 1;
     if (ypml) { yb = __ldg(a.pbE[1] + j); yc = __ldg(a.pcE[1] + j); yik = __ldg(a.ik[1] + j); }
-    const bool xpml = EDGE && act && (i0 < np || i0 + W > a.NxT - np);
+    const bool xpml = EDGE && act && np > 0 && (i0 < np || i0 + W > a.NxT - np);
     // (the gain state is written outside the act-guarded stores: inactive lanes never enter it)
     const bool grow = act && a.gain && j >= a.gj0 && j < a.gj0 + a.gY && i0 + W > a.gi0 && i0 < a.gi0 + a.gX;
     const bool plain_row = act && !ypml && !xpml && i0 >= 1 && i0 + W <= a.NxT;
@@ -1256,7 +1255,7 @@ __device__ __forceinline__ void e_column(const StepArgs<S, T>& a, const SweepGeo
             st_field<SRM>(a, a.Ez, c, ez, 2, src.step);
             if (zpml) { Fld<S, T>::st(a.psiE[1] + zs, pxz); Fld<S, T>::st(a.psiE[2] + zs, pyz); }
             if (ypml) { Fld<S, T>::st(a.psiE[0] + ys, pxy); Fld<S, T>::st(a.psiE[5] + ys, pzy); }
-            if (xpml) xpsi_store<S, T>(a.psiE[3], a.psiE[4], a, k, j, i0, 1, a.NxT, x3, x4);
+            if (xpml) xpsi_store<S, T>(a.psiE[3], a.psiE[4], a, k, j, i0, x3, x4);
         }
 #pragma unroll
         for (int e = 0; e < W; ++e) { hxm[e] = hx[e]; hym[e] = hy[e]; }

@@ -4,12 +4,13 @@
 // three bE coefficient arrays, the 1-D spacing/CPML profiles, psi only inside the PML
 // slabs, the gain block (bounding box of the gain cells: region id, P ping-pong, Nu,
 // Ng), probe series / DFT accumulators and the stability-monitor state.  fdtd_run()
-// issues, per step, k_update_H, k_update_E, the probe/DFT kernel and on monitor steps
+// issues, per step, k_step_fused or k_update_H and k_update_E, the probe/DFT kernel and on monitor steps
 // the FP64 diagnostic reduction, on the handle's stream.  All device memory comes from
 // cudaMalloc at create time (staging for layout transposes on first use).
 #include "../../include/fdtd_b200.h"
 #include "host/outputs.hpp"
 #include "host/waveform.hpp"
+#include "fused.cuh"
 #include "kernels.cuh"
 
 #include <cuda_runtime.h>
@@ -301,7 +302,8 @@ __device__ void block_commit(DiagAccum* acc, double mE, double mP, unsigned fl, 
 // FP64 scans of StabilityMonitor::check_stability (src/stability_monitor.hpp:42-135),
 // calculate_conservation_error (:155-170), compute_integrated_Nu/Ng and
 // compute_polarization_energy (src/two_level_system.hpp:344-418) over the fields after
-// the step.  Field arrays are scanned as flat padded arrays (padding holds zeros).
+// the step.  Field arrays are scanned as flat padded arrays; what lies in a row's padding
+// (cells NxT .. NxP) is skipped: the copy that a fused step wrote holds nothing there.
 template <typename S, typename T, bool FIELDS = true>
 __device__ void monitor_reduce_blocks(const StepArgs<S, T>& a, size_t f0, size_t nflat, const double* __restrict__ dxs,
                                       const double* __restrict__ dys, const double* __restrict__ dzs, int parity_next,
@@ -312,13 +314,21 @@ __device__ void monitor_reduce_blocks(const StepArgs<S, T>& a, size_t f0, size_t
     const size_t stride = size_t(nblk) * blockDim.x;
     // 16-byte vectors: nflat is a multiple of the padded row, itself a multiple of W
     constexpr int W = Vec<T>::W;
+    const int rv = a.NxP / W;  // vectors per row; col: the vector's place in its row
+    const int cstep = int(stride % size_t(rv));
+    int col = int((f0 / W + bid * size_t(blockDim.x) + threadIdx.x) % size_t(rv)) - cstep;
     for (size_t v = f0 / W + bid * size_t(blockDim.x) + threadIdx.x; FIELDS && v < nflat / W; v += stride) {
+        col += cstep;
+        if (col >= rv) col -= rv;
+        const int left = a.NxT - col * W;  // cells of the vector inside the grid
+        if (left <= 0) continue;
         const size_t t = v * W;
         T ex[W], ey[W], ez[W], hx[W], hy[W], hz[W];
         Fld<S, T>::ldg(a.Ex + t, ex); Fld<S, T>::ldg(a.Ey + t, ey); Fld<S, T>::ldg(a.Ez + t, ez);
         Fld<S, T>::ldg(a.Hx + t, hx); Fld<S, T>::ldg(a.Hy + t, hy); Fld<S, T>::ldg(a.Hz + t, hz);
 #pragma unroll
         for (int e = 0; e < W; ++e) {
+            if (e >= left) break;
             const double x = double(ex[e]) * es, y = double(ey[e]) * es, z = double(ez[e]) * es;
             if (!isfinite(x) || !isfinite(y) || !isfinite(z)) fl |= 1u;
             else mE = fmax(mE, fmax(fabs(x), fmax(fabs(y), fabs(z))));
@@ -664,10 +674,10 @@ public:
     void set_timing(int mode) override;
     void set_path(int path) override {
         if (path < 0 || path > 2)
-            throw Failure(FDTD_ERR_INVALID, "kernel path must be 1 (two sweeps) or 2 (slab-ordered step)");
+            throw Failure(FDTD_ERR_INVALID, "kernel path must be 1 (default step) or 2 (slab-ordered step)");
         if (path == 0)
             throw Failure(FDTD_ERR_UNSUPPORTED,
-                          "kernel path 0 (one fused H+E launch per step) is not built: it measured slower than the two sweeps");
+                          "kernel path 0 is reserved");
         if (steps != 0) throw Failure(FDTD_ERR_INVALID, "the kernel path can only change before the first step");
         path_ = path;
     }
@@ -845,13 +855,35 @@ private:
         return hpipe_ ? k_update_H<S, T, true, 0> : k_update_H<S, T, false, 0>;
     }
     // event timing: ev_[0..3] bracket H, E and the auxiliary kernels of one step
-    // kernel path 1 (default): k_update_H + k_update_E in place; path 2: k_step_slabs.
+    // kernel path 1 (default): k_step_fused, or k_update_H + k_update_E in place; path 2: k_step_slabs.
     int path_ = 1;
-    S* fld_[6] = {};
     int xoff_ = 0;  // the field arrays start xoff_ elements into their allocation
-    S* psiH_[6] = {};
-    size_t psi_sz_[6] = {};
-    void point_args_at();
+    // The fields (six arrays, fstride_ elements apart) and psi_H (psi_off_): the current copy,
+    // and while a run takes fused steps the other one.
+    struct FieldCopy {
+        S* f = nullptr;
+        S* psi = nullptr;
+    };
+    FieldCopy cur_{}, other_{};
+    size_t fstride_ = 0, psi_off_[6] = {}, psi_len_ = 0;
+    S* fld(int c) const { return cur_.f + size_t(c) * fstride_ + xoff_; }
+    void point_args_at(StepArgs<S, T>& a, const FieldCopy& f) const {
+        S** const d[6] = {&a.Ex, &a.Ey, &a.Ez, &a.Hx, &a.Hy, &a.Hz};
+        for (int c = 0; c < 6; ++c) *d[c] = f.f + size_t(c) * fstride_ + xoff_;
+        for (int q = 0; q < 6; ++q) a.psiH[q] = f.psi ? f.psi + psi_off_[q] : nullptr;
+    }
+    FieldCopy alloc_copy(bool zero);
+    void free_copy(FieldCopy& f);
+    // One launch per step (fused.cuh): possible for this solve, its tiles, the tensor maps of the
+    // copies ([copy read: 0 cur_ at the run's start, 1 other_][E, H]).
+    bool fusable_ = false;
+    FusedGeom fgeom_{};
+    CUtensorMap maps_[2][2];
+    const S* mapped_[2] = {};
+    void setup_fused();
+    bool begin_fused();
+    void end_fused(uint64_t steps_run);
+    void step_fused(const ESrc& src, int from);
     void pec_faces();  // PECBoundary after the E sweep: the faces of the planes this grid owns
     int timing_ = FDTD_TIMING_OFF;
     cudaEvent_t ev_[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -996,13 +1028,31 @@ Solver<S, T>::Solver(const fdtd_setup_v1& s, int dev, const ShardSpec* shard, bo
     a.kH1 = std::min(shard_.own1, shard_.NzG - 1 - shard_.kz0);
     a.kE0 = std::max(shard_.own0, 1 - shard_.kz0);
     a.kE1 = shard_.own1;
+    // A whole single solve in FP32 or FP64 may step with one fused launch: it needs the row-indexed
+    // material (known below) and the pool (its second copy of the fields is a workspace of each
+    // run).  The switches that shape the two sweeps select the two sweeps.
+    fusable_ = std::is_same_v<S, T> && !shard && !pooled && pooled_;
+    for (const char* v : {"FDTD_B200_LANES", "FDTD_B200_KCHUNK", "FDTD_B200_H_PIPE", "FDTD_B200_E_PIPE"})
+        if (std::getenv(v)) fusable_ = false;
     // 16-bit storage: the H sweep's 8-cell interior vectors start at xi0 = np rounded up to 4
     // cells; the field arrays are offset by xoff_ elements so that xi0 (and every interior
     // vector) falls on a 16-byte boundary.  Every kernel addresses them from the offset pointer.
     xoff_ = 0;
     if constexpr (sizeof(S) == 2) xoff_ = int((8 - round_up(size_t(np_), size_t(W)) % 8) % 8);
-    for (int c = 0; c < 6; ++c) fld_[c] = alloc<S>(nflat_ + 8) + xoff_;
-    point_args_at();
+    fstride_ = round_up(nflat_ + 8, 128 / sizeof(S));
+    if (np_ > 0) {
+        // psi slabs: 0 *_y, 1 *_z, 2 *_z, 3 *_x, 4 *_x, 5 *_y
+        const size_t n2 = size_t(2 * np_);
+        const size_t xs = size_t(NzT_) * NyT_ * XSlab(NxT_, np_, W).len, ys = size_t(NzT_) * n2 * NxP_, zs = n2 * NyT_ * NxP_;
+        const size_t sz[6] = {ys, zs, zs, xs, xs, ys};
+        for (int q = 0; q < 6; ++q) {
+            psi_off_[q] = psi_len_;
+            psi_len_ += round_up(sz[q], 128 / sizeof(S));
+        }
+    }
+    cur_ = alloc_copy(true);
+    point_args_at(a, cur_);
+    dev_bytes += (6 * fstride_ + psi_len_) * sizeof(S);
 
     // bH must be uniform and aE = aH = 1 (sigma = 0, mu_r = 1).
     double bH = s.bH_uniform;
@@ -1124,18 +1174,10 @@ Solver<S, T>::Solver(const fdtd_setup_v1& s, int dev, const ShardSpec* shard, bo
         a.pbH[ax] = upload(bHp); a.pcH[ax] = upload(cH);
     }
     // psi slabs
-    const size_t np2 = size_t(2 * np_);
-    for (int q = 0; q < 6; ++q) { a.psiH[q] = nullptr; a.psiE[q] = nullptr; }
+    for (int q = 0; q < 6; ++q) a.psiE[q] = nullptr;
     if (np_ > 0) {
-        const size_t xs = size_t(NzT_) * NyT_ * np2, ys = size_t(NzT_) * np2 * NxP_, zs = np2 * NyT_ * NxP_;
-        // 0 *_y, 1 *_z, 2 *_z, 3 *_x, 4 *_x, 5 *_y
-        const size_t sz[6] = {ys, zs, zs, xs, xs, ys};
-        for (int q = 0; q < 6; ++q) {
-            psi_sz_[q] = sz[q];
-            psiH_[q] = alloc<S>(sz[q]);
-            a.psiE[q] = alloc<S>(sz[q]);
-            a.psiH[q] = psiH_[q];
-        }
+        S* const e = alloc<S>(psi_len_);
+        for (int q = 0; q < 6; ++q) a.psiE[q] = e + psi_off_[q];
     }
 
     // gain block
@@ -1155,16 +1197,19 @@ Solver<S, T>::Solver(const fdtd_setup_v1& s, int dev, const ShardSpec* shard, bo
         if (hi[0] >= 0) {
             has_gain_ = true;
             a.gain = 1;
-            a.gi0 = lo[0]; a.gj0 = lo[1]; a.gk0 = lo[2];
-            a.gX = hi[0] - lo[0] + 1; a.gY = hi[1] - lo[1] + 1; a.gZ = hi[2] - lo[2] + 1;
+            // in x the box is widened to whole vectors of 4 cells (region -1), so that the two-level
+            // state of a field vector is one vector too
+            a.gi0 = lo[0] / 4 * 4; a.gj0 = lo[1]; a.gk0 = lo[2];
+            a.gX = int(round_up(size_t(hi[0] - a.gi0 + 1), 4)); a.gY = hi[1] - lo[1] + 1; a.gZ = hi[2] - lo[2] + 1;
             const size_t ng = size_t(a.gX) * a.gY * a.gZ;
             std::vector<int8_t> reg(ng);
 #pragma omp parallel for schedule(static)
             for (int k = 0; k < a.gZ; ++k)
                 for (int j = 0; j < a.gY; ++j)
                     for (int i = 0; i < a.gX; ++i)
-                        reg[(size_t(k) * a.gY + j) * a.gX + i] = int8_t(
-                            s.tls_region_map[(size_t(i + a.gi0) * NyT_ + (j + a.gj0)) * NzT_ + (k + a.gk0)]);
+                        reg[(size_t(k) * a.gY + j) * a.gX + i] =
+                            i + a.gi0 < NxT_ ? int8_t(s.tls_region_map[(size_t(i + a.gi0) * NyT_ + (j + a.gj0)) * NzT_ + (k + a.gk0)])
+                                             : int8_t(-1);
             a.greg = upload(reg);
             a.P0 = alloc<T>(ng); a.P1 = alloc<T>(ng); a.Nu = alloc<T>(ng); a.Ng = alloc<T>(ng);
             std::vector<GainCoef<T>> gc(s.n_tls_regions);
@@ -1283,8 +1328,177 @@ Solver<S, T>::Solver(const fdtd_setup_v1& s, int dev, const ShardSpec* shard, bo
     if (gyE > 65535) throw Failure(FDTD_ERR_INVALID, "grid too large for the sweep launch shape (NyT)");
     gridH_ = dim3(gxH, gyE, std::max(1, (a.kH1 + kchunkH_ - 1) / kchunkH_));
     gridE_ = dim3(gxE, gyE, std::max(1, (a.kE1 + kchunkE_ - 1) / kchunkE_));
+    if constexpr (std::is_same_v<S, T>) {
+        if (fusable_) setup_fused();
+    }
     if (const char* p = std::getenv("FDTD_B200_KERNEL_PATH")) set_path(std::atoi(p));
     ck(cudaStreamSynchronize(st_), "setup upload");
+}
+
+// The fused step's tiles and chunks, and whether the solve takes it.
+template <typename S, typename T>
+void Solver<S, T>::setup_fused() {
+    using F = FusedShape<T>;
+    constexpr int W = F::W;
+    FusedGeom& f = fgeom_;
+    f.nrow = int(mat_rows_);
+    f.nzero = -0.0f;
+    const int nv = (NxT_ + W - 1) / W;
+    f.gx = (nv + F::kMaxU - 1) / F::kMaxU;
+    f.u = int(round_up(size_t((nv + f.gx - 1) / f.gx), F::kAlignU));
+    f.gy = (NyT_ + F::TY - 1) / F::TY;
+    // Planes per chunk: a chunk recomputes one plane and fills its ring once, about 3 planes'
+    // time, and the last blocks run alone for half a chunk; with fewer blocks than slots a
+    // chunk's own length is the time.
+    const double slots = 2 * 148, ntile = double(f.gx) * f.gy;
+    double best = 1e300;
+    for (int kc = 1; kc <= std::min(NzT_, int(F::kMaxKc)); ++kc) {
+        const double nb = ntile * ((NzT_ + kc - 1) / kc);
+        const double cost = nb <= slots ? kc + 3 : nb / slots * (kc + 3) + 0.5 * (kc + 3);
+        if (cost < best) { best = cost; f.kc = kc; }
+    }
+    // Which solves: a tile row takes a warp whatever it owns, so a row's vectors must fill most of
+    // its tiles (four fifths of 30 each), and the grid must be large enough that the second
+    // read of E and H would come from HBM (FP64, whose arithmetic is a larger share: 6 M cells) or,
+    // in FP32, that the fuller launch pays for a block's longer start (1 M).  Two sweeps -> fused,
+    // us per step, cubes with 10 - 12 CPML cells and gain unless noted: FP32 100^3 46 -> 41, 200^3
+    // 193 -> 185, 400^3 1025 -> 910, 536^3 2160 -> 1880; but 64^3 25 -> 26, and where tiles are
+    // less full 150^3 (0.63) 89 -> 122, 280^3 (0.78) 375 -> 398.  FP64 200^3 296 -> 281, 280^3
+    // 683 -> 606, 400^3 1820 -> 1529, 536^3 4250 -> 3360; but 150^3 170 -> 173, 201x201x69
+    // 137 -> 158.  FDTD_B200_FUSED = 0 / 1: never / wherever possible.
+    const double cells = double(NxT_) * NyT_ * NzT_;
+    bool take = 5 * nv >= 4 * F::kMaxU * f.gx && cells >= (sizeof(T) == 8 ? 6e6 : 1e6);
+    if (const char* e = std::getenv("FDTD_B200_FUSED")) take = std::string(e) != "0";
+    // psi is addressed with 32-bit offsets
+    const size_t xs = size_t(NzT_) * NyT_ * XSlab(NxT_, np_, W).len, ys = size_t(NzT_) * 2 * np_ * NxP_,
+                 zs = size_t(2 * np_) * NyT_ * NxP_;
+    fusable_ = take && a_.bidx != nullptr && std::max({xs, ys, zs, plane_}) < (size_t(1) << 31) && f.gy <= 65535 &&
+               (NzT_ + f.kc - 1) / f.kc <= 65535;
+    if (!fusable_) return;
+    for (bool sh : {false, true})
+        ck(cudaFuncSetAttribute(fused_kernel<T>(sh), cudaFuncAttributeMaxDynamicSharedMemorySize, int(F::bytes())),
+           "cudaFuncSetAttribute");
+}
+
+template <typename S, typename T>
+typename Solver<S, T>::FieldCopy Solver<S, T>::alloc_copy(bool zero) {
+    FieldCopy f;
+    dev_alloc(reinterpret_cast<void**>(&f.f), 6 * fstride_ * sizeof(S));
+    if (psi_len_) {
+        try {
+            dev_alloc(reinterpret_cast<void**>(&f.psi), psi_len_ * sizeof(S));
+        } catch (...) {
+            dev_free(f.f);
+            throw;
+        }
+    }
+    if (zero) {
+        ck(cudaMemsetAsync(f.f, 0, 6 * fstride_ * sizeof(S), st_), "cudaMemsetAsync");
+        if (f.psi) ck(cudaMemsetAsync(f.psi, 0, psi_len_ * sizeof(S), st_), "cudaMemsetAsync");
+    }
+    return f;
+}
+
+template <typename S, typename T>
+void Solver<S, T>::free_copy(FieldCopy& f) {
+    if (f.f) dev_free(f.f);
+    if (f.psi) dev_free(f.psi);
+    f = FieldCopy{};
+}
+
+// cuTensorMapEncodeTiled from the driver the runtime has loaded (the library is not linked to it).
+using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                 const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled encode_tiled() {
+    static const EncodeTiled fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            p = nullptr;
+        }
+        return reinterpret_cast<EncodeTiled>(p);
+    }();
+    return fn;
+}
+
+// The second copy of the fields for the steps of one run() call, from the stream-ordered pool (it
+// goes back at the call's end, so that between calls a solve holds what it held without it).
+// false: the run takes the two sweeps, in place -- no row-indexed material, or a device so full
+// that the copy would leave less than its own size free for other handles.
+template <typename S, typename T>
+bool Solver<S, T>::begin_fused() {
+    if (!fusable_ || path_ != 1 || timing_ == FDTD_TIMING_KERNELS || !encode_tiled()) return false;
+    const size_t bytes = (6 * fstride_ + psi_len_) * sizeof(S);
+    if (bytes > (size_t(256) << 20)) {
+        size_t free_b = 0, total = 0;
+        ck(cudaMemGetInfo(&free_b, &total), "cudaMemGetInfo");
+        cudaMemPool_t pool;
+        ck(cudaDeviceGetDefaultMemPool(&pool, device), "cudaDeviceGetDefaultMemPool");
+        uint64_t held = 0, used = 0;  // what the pool keeps for reuse is free too
+        ck(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held), "cudaMemPoolGetAttribute");
+        ck(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used), "cudaMemPoolGetAttribute");
+        if (free_b + (held - std::min(held, used)) < 2 * bytes) return false;
+    }
+    try {
+        other_ = alloc_copy(false);
+    } catch (const Failure& f) {
+        if (f.code != FDTD_ERR_OOM) throw;
+        cudaGetLastError();
+        return false;
+    }
+    using F = FusedShape<T>;
+    const FieldCopy* const cp[2] = {&cur_, &other_};
+    for (int b = 0; b < 2; ++b) {
+        if (mapped_[b] == cp[b]->f) continue;
+        const CUtensorMapDataType type =
+            std::is_same_v<T, double> ? CU_TENSOR_MAP_DATA_TYPE_FLOAT64 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+        const cuuint64_t dim[4] = {cuuint64_t(NxT_), cuuint64_t(NyT_), cuuint64_t(NzT_), 3};
+        const cuuint64_t stride[3] = {NxP_ * sizeof(S), plane_ * sizeof(S), fstride_ * sizeof(S)};
+        const cuuint32_t one[4] = {1, 1, 1, 1};
+        for (int h = 0; h < 2; ++h) {
+            const cuuint32_t box[4] = {cuuint32_t(F::XW), cuuint32_t(F::TY + 2 - h), 1, 3};
+            const CUresult r = encode_tiled()(&maps_[b][h], type, 4, cp[b]->f + 3 * size_t(h) * fstride_, dim, stride, box,
+                                              one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+                                              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+            if (r != CUDA_SUCCESS) {
+                free_copy(other_);
+                mapped_[0] = mapped_[1] = nullptr;
+                throw Failure(FDTD_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+            }
+        }
+        mapped_[b] = cp[b]->f;
+    }
+    return true;
+}
+
+// The copy that holds the fields after `n` of the run's steps stays, the other goes back.
+template <typename S, typename T>
+void Solver<S, T>::end_fused(uint64_t n) {
+    if (n & 1) {
+        std::swap(cur_, other_);
+        std::swap(mapped_[0], mapped_[1]);
+        std::swap(maps_[0], maps_[1]);
+    }
+    free_copy(other_);
+    point_args_at(a_, cur_);
+}
+
+// One step from copy `from` (0 cur_, 1 other_) to the other; a_ then describes the latter.
+template <typename S, typename T>
+void Solver<S, T>::step_fused(const ESrc& src, int from) {
+    if constexpr (std::is_same_v<S, T>) {
+        using F = FusedShape<T>;
+        PsiOld<T> old;
+        for (int q = 0; q < 6; ++q) old.p[q] = a_.psiH[q];
+        point_args_at(a_, from ? cur_ : other_);
+        const dim3 grid(unsigned(fgeom_.gx), unsigned(fgeom_.gy), unsigned((NzT_ + fgeom_.kc - 1) / fgeom_.kc));
+        fused_kernel<T>(src.ns != 0)<<<grid, dim3(32, F::kWarps), F::bytes(), st_>>>(maps_[from][0], maps_[from][1], a_, old,
+                                                                                    fgeom_, src, d_status_);
+        ++launches;
+    }
 }
 
 template <typename S, typename T>
@@ -1327,12 +1541,6 @@ void Solver<S, T>::pec_faces() {
 }
 
 template <typename S, typename T>
-void Solver<S, T>::point_args_at() {
-    a_.Ex = fld_[0]; a_.Ey = fld_[1]; a_.Ez = fld_[2];
-    a_.Hx = fld_[3]; a_.Hy = fld_[4]; a_.Hz = fld_[5];
-}
-
-template <typename S, typename T>
 void Solver<S, T>::set_timing(int mode) {
     if (mode < FDTD_TIMING_OFF || mode > FDTD_TIMING_KERNELS) throw Failure(FDTD_ERR_INVALID, "bad timing mode");
     ck(cudaSetDevice(device), "cudaSetDevice");
@@ -1362,6 +1570,8 @@ Solver<S, T>::~Solver() {
         if (trec_ev_[q]) cudaEventDestroy(trec_ev_[q]);
     for (auto& e : ev_) if (e) cudaEventDestroy(e);
     for (void* p : ptrs_) dev_free(p);
+    free_copy(cur_);
+    free_copy(other_);
     if (d_stage_) dev_free(d_stage_);
     if (d_series_) dev_free(d_series_);
     if (st_) cudaStreamDestroy(st_);
@@ -1507,14 +1717,14 @@ void Solver<S, T>::from_device(const D* src, double* h, double scale) {
 template <typename S, typename T>
 void Solver<S, T>::set_field(int comp, const double* h) {
     if (comp < 0 || comp > 5) throw Failure(FDTD_ERR_INVALID, "component must be 0..5");
-    to_device(h, fld_[comp], 1.0 / (comp < 3 ? sE_ : sH_));
+    to_device(h, fld(comp), 1.0 / (comp < 3 ? sE_ : sH_));
     ck(cudaStreamSynchronize(st_), "set_field");
 }
 
 template <typename S, typename T>
 void Solver<S, T>::get_field(int comp, double* h) {
     if (comp < 0 || comp > 5) throw Failure(FDTD_ERR_INVALID, "component must be 0..5");
-    from_device(fld_[comp], h, comp < 3 ? sE_ : sH_);
+    from_device(fld(comp), h, comp < 3 ? sE_ : sH_);
 }
 
 template <typename S, typename T>
@@ -1579,6 +1789,12 @@ void Solver<S, T>::run(uint64_t n) {
     src_static(src);
     const int pthreads = int(nprobes_ * std::max<uint32_t>(nf_, 1));
     const bool per_kernel = timing_ == FDTD_TIMING_KERNELS;
+    const bool fused = n > 0 && begin_fused();
+    struct Other {  // the workspace goes back whichever way the run ends
+        Solver* s;
+        uint64_t n = 0;
+        ~Other() { if (s) s->end_fused(n); }
+    } other{fused ? this : nullptr};
     if (timing_ == FDTD_TIMING_RUN) ck(cudaEventRecord(ev_[0], st_), "cudaEventRecord");
     for (uint64_t s = n0; s < last; ++s) {
         src_step(src, s);
@@ -1593,6 +1809,9 @@ void Solver<S, T>::run(uint64_t n) {
             slabs<<<gridS_, blk, 0, st_>>>(a_, src, geom_, plan_, d_ctr_, d_status_);
             if (per_kernel) ck(cudaEventRecord(ev_[1], st_), "cudaEventRecord");
             launches += 1;
+        } else if (fused) {
+            step_fused(src, int((s - n0) & 1));
+            other.n = s + 1 - n0;
         } else {
             h_kernel()<<<gridH_, blk, hpipe_ ? HPipe<S>::bytes() : 0, st_>>>(a_, kchunkH_, geom_, src.step);
             if (per_kernel) ck(cudaEventRecord(ev_[1], st_), "cudaEventRecord");
@@ -1646,6 +1865,7 @@ void Solver<S, T>::run(uint64_t n) {
         MonitorState ms{};
         ck(cudaMemcpy(&ms, d_ms_, sizeof(ms), cudaMemcpyDeviceToHost), "monitor state");
         steps = ms.step + 1;
+        other.n = steps - n0;  // the launches after the failed monitor step did nothing
         series_count_ = std::min<uint64_t>(series_count_, (steps + save_every_ - 1) / save_every_);
         if (writer_) write_point_samples();
         throw Failure(FDTD_ERR_UNSTABLE, "stability monitor stopped the solve at step " + std::to_string(ms.step));
