@@ -41,72 +41,6 @@ __device__ __forceinline__ void tma_load4(void* dst, const CUtensorMap* m, int x
         : "memory");
 }
 
-// Arithmetic of a whole vector, every operation rounded on its own: FP32 in pairs (one instruction
-// for two cells, the same rounding).
-__device__ __forceinline__ unsigned long long pair(float x, float y) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ void unpair(unsigned long long r, float& x, float& y) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(r));
-}
-__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-// a * b as a * b + (-0): the same value for every a and b.  A plain mul.rn.f32x2 whose result feeds a
-// subtraction is contracted with it by the assembler, explicit rounding or not; nz = (-0, -0) is a
-// kernel argument so that it cannot tell.
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b, unsigned long long nz) {
-    return fma2(a, b, nz);
-}
-// r = (b - a) * s
-__device__ __forceinline__ void vdq(float (&r)[4], const float (&b)[4], const float (&a)[4], float s, float nz) {
-    const unsigned long long s2 = pair(s, s), z2 = pair(nz, nz);
-#pragma unroll
-    for (int e = 0; e < 4; e += 2)
-        unpair(mul2(sub2(pair(b[e], b[e + 1]), pair(a[e], a[e + 1])), s2, z2), r[e], r[e + 1]);
-}
-__device__ __forceinline__ void vdq(double (&r)[2], const double (&b)[2], const double (&a)[2], double s, float) {
-#pragma unroll
-    for (int e = 0; e < 2; ++e) r[e] = dq(b[e], a[e], s);
-}
-// r *= s, cell by cell
-__device__ __forceinline__ void vmul(float (&r)[4], const float (&s)[4], float nz) {
-#pragma unroll
-    for (int e = 0; e < 4; e += 2) unpair(mul2(pair(r[e], r[e + 1]), pair(s[e], s[e + 1]), pair(nz, nz)), r[e], r[e + 1]);
-}
-__device__ __forceinline__ void vmul(double (&r)[2], const double (&s)[2], float) {
-#pragma unroll
-    for (int e = 0; e < 2; ++e) r[e] = mul_rn(r[e], s[e]);
-}
-// r -= b
-__device__ __forceinline__ void vsub(float (&r)[4], const float (&b)[4]) {
-#pragma unroll
-    for (int e = 0; e < 4; e += 2) unpair(sub2(pair(r[e], r[e + 1]), pair(b[e], b[e + 1])), r[e], r[e + 1]);
-}
-__device__ __forceinline__ void vsub(double (&r)[2], const double (&b)[2]) {
-#pragma unroll
-    for (int e = 0; e < 2; ++e) r[e] = sub_rn(r[e], b[e]);
-}
-// r = b * c + r
-__device__ __forceinline__ void vfma(float (&r)[4], const float (&b)[4], const float (&c)[4]) {
-#pragma unroll
-    for (int e = 0; e < 4; e += 2)
-        unpair(fma2(pair(b[e], b[e + 1]), pair(c[e], c[e + 1]), pair(r[e], r[e + 1])), r[e], r[e + 1]);
-}
-__device__ __forceinline__ void vfma(double (&r)[2], const double (&b)[2], const double (&c)[2]) {
-#pragma unroll
-    for (int e = 0; e < 2; ++e) r[e] = fma_rn(b[e], c[e], r[e]);
-}
-
 // Keeps a value in its register: the compiler may not load it again where it is used.
 __device__ __forceinline__ void opaque(float& v) { asm volatile("" : "+f"(v)); }
 __device__ __forceinline__ void opaque(double& v) { asm volatile("" : "+d"(v)); }
@@ -199,38 +133,11 @@ __device__ __forceinline__ void psi_x(T (&d)[Vec<T>::W], T (&psi)[Vec<T>::W], co
         prefetch_l2(po + (q + step));
     }
 }
-// v[e] += b[e] * c[e] rounded once, in the cells of mask m (all of them unless MASKED).
-template <bool MASKED, typename T>
-__device__ __forceinline__ void update(T (&v)[Vec<T>::W], const T (&b)[Vec<T>::W], const T (&c)[Vec<T>::W], unsigned m) {
-    if constexpr (MASKED) {
-        T n[Vec<T>::W];
-#pragma unroll
-        for (int e = 0; e < Vec<T>::W; ++e) n[e] = v[e];
-        vfma(n, b, c);
-#pragma unroll
-        for (int e = 0; e < Vec<T>::W; ++e) v[e] = (m >> e) & 1u ? n[e] : v[e];
-    } else {
-        vfma(v, b, c);
-    }
-}
-
-// Current of the step's sources into component comp at cell (i, j, k): the point sources, then the sheets.
-template <bool SH, typename T>
-__device__ __forceinline__ T source_J(const ESrc& src, int comp, int i, int j, int k) {
-    T J = 0;
-    for (int s = 0; s < src.n; ++s)
-        if (src.sc[s] == comp && src.si[s] == i && src.sj[s] == j && src.sk[s] == k) J = add_rn(J, T(src.J[s]));
-    if constexpr (SH) {
-        T Jx = comp == 0 ? J : T(0), Jy = comp == 1 ? J : T(0), Jz = comp == 2 ? J : T(0);
-        sheet_J(src, i, j, k, Jx, Jy, Jz);
-        J = comp == 0 ? Jx : comp == 1 ? Jy : Jz;
-    }
-    return J;
-}
-template <bool SH, typename T>
-__device__ __forceinline__ void sub_J(const ESrc& src, int comp, int x0, int j, int k, T (&c)[Vec<T>::W]) {
-#pragma unroll
-    for (int e = 0; e < Vec<T>::W; ++e) c[e] = sub_rn(c[e], source_J<SH, T>(src, comp, x0 + e, j, k));
+// v += b * c, rounded once, in the cells of mask m (all of them unless MASKED).
+template <bool MASKED, typename T, int W>
+__device__ __forceinline__ void update(T (&v)[W], const T (&b)[W], const T (&c)[W], unsigned m) {
+    if constexpr (MASKED) vfma_in(v, b, c, m);
+    else vfma(v, b, c);
 }
 
 // a: the arguments with the fields and psi_H of the copy being written.
@@ -394,19 +301,19 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
             Vec<T>::ld(xco, idx);
             // Hx: dEz/dy - dEy/dz
             Vec<T>::ld(eprev + XW + 2 * EC, t);
-            vdq(da, t, ez, idy, g.nzero);
+            vdq(da, t, ez, idy);
             Vec<T>::ld(ecur + EC, t);
-            vdq(db, t, ey, idz, g.nzero);
+            vdq(db, t, ey, idz);
             if (G && ypml) psi_yz(da, old.p[0], a.psiH[0], yq, ys1, in, mine, yc + 1, yc[5], a.psc);
             if (G && zpml) psi_yz(db, old.p[1], a.psiH[1], zq, zs, in, mine, zc + 1, zc[5], a.psc);
             vsub(da, db);
             update<G>(hx, nbH, da, mh);
             // Hy: dEx/dz - dEz/dx
             Vec<T>::ld(ecur, t);
-            vdq(da, t, ex, idz, g.nzero);
+            vdq(da, t, ex, idz);
 #pragma unroll
             for (int e = 0; e < W; ++e) db[e] = sub_rn((e < W - 1) ? ez[e + 1] : ezn, ez[e]);
-            vmul(db, idx, g.nzero);
+            vmul(db, idx);
             if (G && zpml) psi_yz(da, old.p[2], a.psiH[2], zq, zs, in, mine, zc + 1, zc[5], a.psc);
             if (G && xgen) psi_x(db, px0, old.p[3], a.psiH[3], xq, xs1, xpml && mine, xco + XW, xco + 2 * XW, xco + 5 * XW, mx, a.psc);
             vsub(da, db);
@@ -415,8 +322,8 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
             Vec<T>::ld(eprev + XW, t);
 #pragma unroll
             for (int e = 0; e < W; ++e) da[e] = sub_rn((e < W - 1) ? ey[e + 1] : eyn, ey[e]);
-            vmul(da, idx, g.nzero);
-            vdq(db, t, ex, idy, g.nzero);
+            vmul(da, idx);
+            vdq(db, t, ex, idy);
             if (G && xgen) psi_x(da, px1, old.p[4], a.psiH[4], xq, xs1, xpml && mine, xco + XW, xco + 2 * XW, xco + 5 * XW, mx, a.psc);
             if (G && ypml) psi_yz(db, old.p[5], a.psiH[5], yq, ys1, in, mine, yc + 1, yc[5], a.psc);
             vsub(da, db);
@@ -461,18 +368,18 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
             Vec<T>::ld(xco, idx);
             // Ex: dHz/dy - dHy/dz
             Vec<T>::ld(xs + 2 * HC, t);
-            vdq(da, hz, t, idy, g.nzero);
-            vdq(db, hy, hym, idz, g.nzero);
+            vdq(da, hz, t, idy);
+            vdq(db, hy, hym, idz);
             if (G && ypml) psi_yz(da, a.psiE[0], a.psiE[0], yq, ys1, own, own, yc + 3, yc[5], a.psc);
             if (G && zpml) psi_yz(db, a.psiE[1], a.psiE[1], zq, zs, own, own, zc + 3, zc[5], a.psc);
             vsub(da, db);
             if (G && special) sub_J<SH>(src, 0, x0, j, k, da);
             update<G>(ex, bx, da, me);
             // Ey: dHx/dz - dHz/dx
-            vdq(da, hx, hxm, idz, g.nzero);
+            vdq(da, hx, hxm, idz);
 #pragma unroll
             for (int e = 0; e < W; ++e) db[e] = sub_rn(hz[e], (e > 0) ? hz[e - 1] : hzp);
-            vmul(db, idx, g.nzero);
+            vmul(db, idx);
             if (G && zpml) psi_yz(da, a.psiE[2], a.psiE[2], zq, zs, own, own, zc + 3, zc[5], a.psc);
             if (G && xgen) psi_x(db, px0, a.psiE[3], a.psiE[3], xq, xs1, xpml && own, xco + 3 * XW, xco + 4 * XW, xco + 5 * XW, mx, a.psc);
             vsub(da, db);
@@ -482,60 +389,14 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
             Vec<T>::ld(xs, t);
 #pragma unroll
             for (int e = 0; e < W; ++e) da[e] = sub_rn(hy[e], (e > 0) ? hy[e - 1] : hyp);
-            vmul(da, idx, g.nzero);
-            vdq(db, hx, t, idy, g.nzero);
+            vmul(da, idx);
+            vdq(db, hx, t, idy);
             if (G && xgen) psi_x(da, px1, a.psiE[4], a.psiE[4], xq, xs1, xpml && own, xco + 3 * XW, xco + 4 * XW, xco + 5 * XW, mx, a.psc);
             if (G && ypml) psi_yz(db, a.psiE[5], a.psiE[5], yq, ys1, own, own, yc + 3, yc[5], a.psc);
             vsub(da, db);
             if (G && special) sub_J<SH>(src, 2, x0, j, k, da);
             if (G && grow && k >= a.gk0 && k < a.gk0 + a.gZ) {
-                // the two-level state of the vector (the gain box is W-aligned, region -1 = no gain)
-                T* const Pcur = src.parity ? a.P1 : a.P0;
-                T* const Pold = src.parity ? a.P0 : a.P1;  // holds P^{n-1}, receives P^{n+1}
-                const size_t gq = (size_t(k - a.gk0) * a.gY + (j - a.gj0)) * a.gX + (x0 - a.gi0);
-                int reg[W];
-                T P[W], Pp[W], Nu[W], Ng[W];
-#pragma unroll
-                for (int e = 0; e < W; ++e) reg[e] = a.greg[gq + e];
-                Vec<T>::ld(Pcur + gq, P); Vec<T>::ld(Pold + gq, Pp);
-                Vec<T>::ld(a.Nu + gq, Nu); Vec<T>::ld(a.Ng + gq, Ng);
-#pragma unroll
-                for (int e = 0; e < W; ++e) {
-                    if (!((me >> e) & 1u)) continue;
-                    if (reg[e] >= 0 && a.gcoef[reg[e]].active) {
-                        // polarization with E^n, E update with -dP/dt, populations with E^{n+1}
-                        const GainCoef<T>& q = a.gcoef[reg[e]];
-                        const T ez_old = ez[e];
-                        const T ng_frac = mul_rn(sub_rn(Ng[e], Nu[e]), q.inv_N0);
-                        const T Pn = fma_rn(q.pa3, Pp[e], fma_rn(q.pa2, P[e], mul_rn(q.kapaN0, mul_rn(ng_frac, ez_old))));
-                        const T dPn = sub_rn(Pn, P[e]);
-                        const T dP = mul_rn(dPn, q.inv_dt);
-                        ez[e] = fma_rn(bz[e], sub_rn(da[e], mul_rn(dP, q.dp_scale)), ez[e]);
-                        const T e_avg = mul_rn(T(0.5), add_rn(ez[e], ez_old));
-                        const T stim = mul_rn(mul_rn(mul_rn(e_avg, dPn), q.inv_dt), q.inv_hbar_omega);
-                        T dNu = fma_rn(-q.inv_tau, Nu[e], stim);
-                        T dNg = fma_rn(q.inv_tau, Nu[e], -stim);
-                        if (q.pump != T(0)) { dNu = fma_rn(q.pump, Ng[e], dNu); dNg = fma_rn(-q.pump, Ng[e], dNg); }
-                        T nu = fma_rn(q.dt, dNu, Nu[e]);
-                        T ng = fma_rn(q.dt, dNg, Ng[e]);
-                        nu = fmax(T(0), nu);
-                        ng = fmax(T(0), ng);
-                        if (q.clamp) {
-                            const T tot = add_rn(nu, ng);
-                            if (tot > T(1e-30)) { const T f = div_rn(q.N0, tot); nu = mul_rn(nu, f); ng = mul_rn(ng, f); }
-                            nu = fmin(nu, q.N0);
-                            ng = sub_rn(q.N0, nu);
-                        }
-                        Pp[e] = Pn;
-                        Nu[e] = nu;
-                        Ng[e] = ng;
-                    } else {
-                        ez[e] = fma_rn(bz[e], da[e], ez[e]);
-                    }
-                }
-                Vec<T>::st(Pold + gq, Pp);
-                Vec<T>::st(a.Nu + gq, Nu);
-                Vec<T>::st(a.Ng + gq, Ng);
+                gain_vector(a, src.parity, x0, j, k, me, da, bz, ez);
             } else {
                 update<G>(ez, bz, da, me);
             }

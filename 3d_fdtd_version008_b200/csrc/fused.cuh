@@ -46,7 +46,6 @@ struct FusedGeom {
     int gx, gy;  // tiles in x, in y
     int kc;      // planes per chunk
     int nrow;    // material rows
-    float nzero; // -0 (fused.cu: mul2)
 };
 
 template <typename T>

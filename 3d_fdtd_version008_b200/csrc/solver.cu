@@ -1342,7 +1342,6 @@ void Solver<S, T>::setup_fused() {
     constexpr int W = F::W;
     FusedGeom& f = fgeom_;
     f.nrow = int(mat_rows_);
-    f.nzero = -0.0f;
     const int nv = (NxT_ + W - 1) / W;
     f.gx = (nv + F::kMaxU - 1) / F::kMaxU;
     f.u = int(round_up(size_t((nv + f.gx - 1) / f.gx), F::kAlignU));
@@ -1358,16 +1357,17 @@ void Solver<S, T>::setup_fused() {
         if (cost < best) { best = cost; f.kc = kc; }
     }
     // Which solves: a tile row takes a warp whatever it owns, so a row's vectors must fill most of
-    // its tiles (four fifths of 30 each), and the grid must be large enough that the second
-    // read of E and H would come from HBM (FP64, whose arithmetic is a larger share: 6 M cells) or,
-    // in FP32, that the fuller launch pays for a block's longer start (1 M).  Two sweeps -> fused,
-    // us per step, cubes with 10 - 12 CPML cells and gain unless noted: FP32 100^3 46 -> 41, 200^3
-    // 193 -> 185, 400^3 1025 -> 910, 536^3 2160 -> 1880; but 64^3 25 -> 26, and where tiles are
-    // less full 150^3 (0.63) 89 -> 122, 280^3 (0.78) 375 -> 398.  FP64 200^3 296 -> 281, 280^3
-    // 683 -> 606, 400^3 1820 -> 1529, 536^3 4250 -> 3360; but 150^3 170 -> 173, 201x201x69
-    // 137 -> 158.  FDTD_B200_FUSED = 0 / 1: never / wherever possible.
+    // its tiles (four fifths of 30 each); and a CPML slab costs the fused step more (its psi is
+    // loaded within a warp's plane, and one x-slab vector slows its whole row segment), so that
+    // the grid must be large enough for the saved HBM bytes to outweigh it.  Two sweeps -> fused, us
+    // per step, cubes with 10 - 12 CPML cells and gain unless noted: FP32 320^3 544 -> 511, 400^3
+    // 945 -> 916, 300x200x500 without gain 521 -> 486, 536^3 2162 -> 1880; but 200^3 175 -> 187,
+    // 236^3 257 -> 268, and where tiles are less full 280^3 (0.78) 353 -> 401.  FP64 200^3 283 -> 280,
+    // 236^3 437 -> 400, 280^3 663 -> 602, 400^3 1770 -> 1540, 536^3 4257 -> 3360; but 150^3 161 -> 169,
+    // 201x201x69 130 -> 156.  Without CPML (metal box 157x121x93) FP64 74 -> 59.
+    // FDTD_B200_FUSED = 0 / 1: never / wherever possible.
     const double cells = double(NxT_) * NyT_ * NzT_;
-    bool take = 5 * nv >= 4 * F::kMaxU * f.gx && cells >= (sizeof(T) == 8 ? 6e6 : 1e6);
+    bool take = 5 * nv >= 4 * F::kMaxU * f.gx && cells >= (np_ == 0 ? 1e6 : sizeof(T) == 8 ? 8e6 : 2.5e7);
     if (const char* e = std::getenv("FDTD_B200_FUSED")) take = std::string(e) != "0";
     // psi is addressed with 32-bit offsets
     const size_t xs = size_t(NzT_) * NyT_ * XSlab(NxT_, np_, W).len, ys = size_t(NzT_) * 2 * np_ * NxP_,
