@@ -1156,6 +1156,81 @@ __device__ __forceinline__ void h_column8(const StepArgs<S, float>& a, const Swe
     }
 }
 
+struct ProbeDev {
+    long long off;  // device-layout offset of the probe cell
+    int comp;
+};
+
+// Probe value in physical units: stored E and H times their field scales es, hs.
+// get_field_value (src/detectors/idetector.hpp:79-110) on one cell's six FP64 values, with
+// every product and sum rounded on its own (no contraction), as the reference computes it.
+__device__ __forceinline__ double component_value(int comp, double ex, double ey, double ez, double hx, double hy,
+                                                  double hz) {
+    auto cross = [](double a, double b, double c, double d) { return __dsub_rn(__dmul_rn(a, b), __dmul_rn(c, d)); };
+    auto norm = [](double x, double y, double z) {
+        return sqrt(__dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z)));
+    };
+    switch (comp) {
+        case 0: return ex;
+        case 1: return ey;
+        case 2: return ez;
+        case 3: return hx;
+        case 4: return hy;
+        case 5: return hz;
+        case 6: return norm(ex, ey, ez);
+        case 7: return norm(hx, hy, hz);
+        case 8: return cross(ey, hz, ez, hy);
+        case 9: return cross(ez, hx, ex, hz);
+        case 10: return cross(ex, hy, ey, hx);
+        case 11: return norm(cross(ey, hz, ez, hy), cross(ez, hx, ex, hz), cross(ex, hy, ey, hx));
+    }
+    return 0.0;
+}
+
+// Point probes after the E update of step n: sample (every save_every steps) and the FP64 DFT
+// accumulation X_m += v * exp(-i 2 pi f_m t) * dt at t = (n+1) dt.
+struct ProbeStep {
+    const ProbeDev* probes;
+    int nprobes, nf;
+    const double* freqs;
+    double *dft, *series;
+    long long sample;       // sample index of this step, or -1
+    double t, dt;
+    double es, hs;          // stored fields are E / es and H / hs
+    unsigned long long step;
+    const unsigned long long* failed_step;  // the step a failed monitor evaluation stopped at
+};
+
+// One (probe, frequency) pair; f: Ex, the other arrays fs elements apart each.
+template <typename S>
+__device__ __forceinline__ void probe_dft_thread(const S* f, long long fs, const ProbeStep& p, int tid) {
+    const int per = p.nf > 0 ? p.nf : 1;
+    if (tid >= p.nprobes * per) return;
+    const int q = tid / per, m = tid % per;
+    const S* o = f + p.probes[q].off;
+    const double v = component_value(p.probes[q].comp, double(to_c(o[0])) * p.es, double(to_c(o[fs])) * p.es,
+                                     double(to_c(o[2 * fs])) * p.es, double(to_c(o[3 * fs])) * p.hs,
+                                     double(to_c(o[4 * fs])) * p.hs, double(to_c(o[5 * fs])) * p.hs);
+    if (m == 0 && p.sample >= 0) p.series[size_t(p.sample) * p.nprobes + q] = v;
+    if (p.nf > 0) {
+        double s, c;
+        sincospi(2.0 * p.freqs[m] * p.t, &s, &c);
+        double* acc = p.dft + 2 * (size_t(q) * p.nf + m);
+        acc[0] = __dadd_rn(acc[0], __dmul_rn(__dmul_rn(v, c), p.dt));
+        acc[1] = __dsub_rn(acc[1], __dmul_rn(__dmul_rn(v, s), p.dt));
+    }
+}
+
+// A block of the H sweep of step n + 1 that records the probes of step n: E holds still during that
+// sweep.  (A call of its own, so that the sweep's registers do not pay for it.)  After a failed
+// monitor step only that step's own probes are still due.
+template <typename S>
+__device__ __noinline__ void probe_block(const S* f, long long fs, const unsigned* status, const ProbeStep& p, int tid, int nt) {
+    if (*status != 0u && *p.failed_step != p.step) return;
+    const int n = p.nprobes * (p.nf > 0 ? p.nf : 1);
+    for (int t = tid; t < n; t += nt) probe_dft_thread(f, fs, p, t);
+}
+
 // One block of the H sweep: block (bx, by, bz) of the solve's launch grid.
 template <typename S, typename T, bool PIPE = false, int SRM = 2>
 __device__ __forceinline__ void update_H_block(const StepArgs<S, T>& a, const int kchunk, const SweepGeom& g,
@@ -1197,6 +1272,18 @@ __device__ __forceinline__ void update_H_block(const StepArgs<S, T>& a, const in
 template <typename S, typename T, bool PIPE = false, int SRM = 2>
 __global__ void __launch_bounds__(32 * kBlockY, 2)
 k_update_H(const StepArgs<S, T> a, const int kchunk, const SweepGeom g, const unsigned step) {
+    update_H_block<S, T, PIPE, SRM>(a, kchunk, g, blockIdx.x, blockIdx.y, blockIdx.z, step);
+}
+// With the last step's probes in one more z layer of blocks (small grids; the call costs the sweep
+// itself 2 % on large ones).
+template <typename S, typename T, bool PIPE = false, int SRM = 2>
+__global__ void __launch_bounds__(32 * kBlockY, 2)
+k_update_H_probe(const StepArgs<S, T> a, const int kchunk, const SweepGeom g, const unsigned step, const ProbeStep probe) {
+    if (blockIdx.z + 1 == gridDim.z) {
+        if (blockIdx.x == 0 && blockIdx.y == 0)
+            probe_block(a.Ex, a.Ey - a.Ex, a.status, probe, threadIdx.y * 32 + threadIdx.x, 32 * kBlockY);
+        return;
+    }
     update_H_block<S, T, PIPE, SRM>(a, kchunk, g, blockIdx.x, blockIdx.y, blockIdx.z, step);
 }
 

@@ -144,37 +144,6 @@ __global__ void k_gain_block(double* __restrict__ full, T* __restrict__ blk, con
     }
 }
 
-struct ProbeDev {
-    long long off;  // device-layout offset of the probe cell
-    int comp;
-};
-
-// Probe value in physical units: stored E and H times their field scales es, hs.
-// get_field_value (src/detectors/idetector.hpp:79-110) on one cell's six FP64 values, with
-// every product and sum rounded on its own (no contraction), as the reference computes it.
-__device__ __forceinline__ double component_value(int comp, double ex, double ey, double ez, double hx, double hy,
-                                                  double hz) {
-    auto cross = [](double a, double b, double c, double d) { return __dsub_rn(__dmul_rn(a, b), __dmul_rn(c, d)); };
-    auto norm = [](double x, double y, double z) {
-        return sqrt(__dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z)));
-    };
-    switch (comp) {
-        case 0: return ex;
-        case 1: return ey;
-        case 2: return ez;
-        case 3: return hx;
-        case 4: return hy;
-        case 5: return hz;
-        case 6: return norm(ex, ey, ez);
-        case 7: return norm(hx, hy, hz);
-        case 8: return cross(ey, hz, ez, hy);
-        case 9: return cross(ez, hx, ex, hz);
-        case 10: return cross(ex, hy, ey, hx);
-        case 11: return norm(cross(ey, hz, ez, hy), cross(ez, hx, ex, hz), cross(ex, hy, ey, hx));
-    }
-    return 0.0;
-}
-
 // FieldMovie2D::record_after_E (src/detectors/field_movie_2d.hpp:107-148): one component on
 // one slice plane, in the reference's order -- XY: (i, j), XZ: (i, k), YZ: (j, k), the
 // second index fastest -- as FP64 or FP32.  One thread per output value.
@@ -198,42 +167,10 @@ __global__ void k_slice(const S* __restrict__ Ex, const S* __restrict__ Ey, cons
     }
 }
 
-template <typename S, typename T>
-__device__ double probe_value(const StepArgs<S, T>& a, const ProbeDev& p, double es, double hs) {
-    const size_t o = size_t(p.off);
-    return component_value(p.comp, double(to_c(a.Ex[o])) * es, double(to_c(a.Ey[o])) * es, double(to_c(a.Ez[o])) * es,
-                           double(to_c(a.Hx[o])) * hs, double(to_c(a.Hy[o])) * hs, double(to_c(a.Hz[o])) * hs);
-}
-
-// Point probes after the E update of step n: sample (every save_every steps) and the
-// FP64 DFT accumulation X_m += v * exp(-i 2 pi f_m t) * dt at t = (n+1) dt.
-// One thread per (probe, frequency).
-template <typename S, typename T>
-__device__ void probe_dft_thread(const StepArgs<S, T>& a, const ProbeDev* __restrict__ probes, int nprobes,
-                                 const double* __restrict__ freqs, int nf, double* __restrict__ dft,
-                                 double* __restrict__ series, long long sample, double t, double dt, double es,
-                                 double hs, int tid) {
-    const int per = nf > 0 ? nf : 1;
-    if (tid >= nprobes * per) return;
-    const int p = tid / per, m = tid % per;
-    const double v = probe_value(a, probes[p], es, hs);
-    if (m == 0 && sample >= 0) series[size_t(sample) * nprobes + p] = v;
-    if (nf > 0) {
-        double s, c;
-        sincospi(2.0 * freqs[m] * t, &s, &c);
-        double* acc = dft + 2 * (size_t(p) * nf + m);
-        acc[0] = __dadd_rn(acc[0], __dmul_rn(__dmul_rn(v, c), dt));
-        acc[1] = __dsub_rn(acc[1], __dmul_rn(__dmul_rn(v, s), dt));
-    }
-}
-
-template <typename S, typename T>
-__global__ void k_probe_dft(const StepArgs<S, T> a, const ProbeDev* __restrict__ probes, int nprobes,
-                            const double* __restrict__ freqs, int nf, double* __restrict__ dft,
-                            double* __restrict__ series, long long sample, double t, double dt, double es, double hs) {
-    if (*a.status) return;
-    probe_dft_thread(a, probes, nprobes, freqs, nf, dft, series, sample, t, dt, es, hs,
-                     int(blockIdx.x * blockDim.x + threadIdx.x));
+template <typename S>
+__global__ void k_probe_dft(const S* f, long long fs, const unsigned* status, const ProbeStep p) {
+    if (*status) return;
+    probe_dft_thread(f, fs, p, int(blockIdx.x * blockDim.x + threadIdx.x));
 }
 
 struct DiagAccum {
@@ -534,8 +471,8 @@ __device__ __forceinline__ void probe_multi_block(int r) {
     const BatchTick& tk = c_btick[r];
     if (*a.status || b.nprobes == 0) return;
     const int n = b.nprobes * (b.nf > 0 ? b.nf : 1);
-    for (int tid = threadIdx.x; tid < n; tid += blockDim.x)
-        probe_dft_thread(a, b.probes, b.nprobes, b.freqs, b.nf, b.dft, b.series, tk.sample, tk.t, b.dt, b.sE, b.sH, tid);
+    const ProbeStep p{b.probes, b.nprobes, b.nf, b.freqs, b.dft, b.series, tk.sample, tk.t, b.dt, b.sE, b.sH, tk.step, nullptr};
+    for (int tid = threadIdx.x; tid < n; tid += blockDim.x) probe_dft_thread(a.Ex, a.Ey - a.Ex, p, tid);
 }
 
 // one block per solve
@@ -810,10 +747,25 @@ private:
     long long mon_t_ = -1;
     bool pop_first_done_ = false;
     ProbeDev* d_probes_ = nullptr;
+    bool probes_E_ = true;  // every probe reads E only
+    ProbeStep probe_step(uint64_t s) const {
+        return ProbeStep{d_probes_, int(nprobes_), int(nf_), d_freqs_, d_dft_, d_series_,
+                         s % save_every_ == 0 ? (long long)(s / save_every_) : -1, double(s + 1) * dt_, dt_, sE_, sH_, s,
+                         &d_ms_->step};
+    }
+    void launch_probes(uint64_t s) {
+        const int n = int(nprobes_ * std::max<uint32_t>(nf_, 1));
+        k_probe_dft<S><<<(n + 127) / 128, 128, 0, st_>>>(a_.Ex, a_.Ey - a_.Ex, d_status_, probe_step(s));
+        ++launches;
+    }
     double *d_freqs_ = nullptr, *d_dft_ = nullptr, *d_series_ = nullptr;
     uint64_t series_cap_ = 0, series_count_ = 0;
     // monitor
     uint32_t interval_ = 0;
+    // one vector per thread on small grids, 8 blocks per SM on large ones
+    unsigned mon_blocks() const {
+        return unsigned(std::clamp<size_t>((nflat_ / Vec<T>::W + 255) / 256, 1, 8 * 148));
+    }
     double *d_dx_ = nullptr, *d_dy_ = nullptr, *d_dz_ = nullptr;
     DiagAccum* d_acc_ = nullptr;
     MonitorState* d_ms_ = nullptr;
@@ -849,6 +801,12 @@ private:
         return k[4 * int(sheets) + 2 * int(a_.bidx != nullptr) + int(pipe_)];
     }
     using HKernel = void (*)(const StepArgs<S, T>, const int, const SweepGeom, const unsigned);
+    using HProbeKernel = void (*)(const StepArgs<S, T>, const int, const SweepGeom, const unsigned, const ProbeStep);
+    HProbeKernel h_probe_kernel() const {
+        if constexpr (std::is_same_v<S, __nv_bfloat16>)
+            if (srm_) return hpipe_ ? k_update_H_probe<S, T, true, 1> : k_update_H_probe<S, T, false, 1>;
+        return hpipe_ ? k_update_H_probe<S, T, true, 0> : k_update_H_probe<S, T, false, 0>;
+    }
     HKernel h_kernel() const {
         if constexpr (std::is_same_v<S, __nv_bfloat16>)
             if (srm_) return hpipe_ ? k_update_H<S, T, true, 1> : k_update_H<S, T, false, 1>;
@@ -1133,9 +1091,12 @@ Solver<S, T>::Solver(const fdtd_setup_v1& s, int dev, const ShardSpec* shard, bo
     if (const char* e = std::getenv("FDTD_B200_H_PIPE")) hpipe_ = std::string(e) != "0";
     if (const char* e = std::getenv("FDTD_B200_E_PIPE")) pipe_ = a.bidx != nullptr && std::string(e) != "0";
     srm_ = std::is_same_v<S, __nv_bfloat16> && s.rounding == FDTD_ROUND_STOCHASTIC ? 1 : 0;
-    if (hpipe_)
+    if (hpipe_) {
         ck(cudaFuncSetAttribute(h_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, int(HPipe<S>::bytes())),
            "cudaFuncSetAttribute");
+        ck(cudaFuncSetAttribute(h_probe_kernel(), cudaFuncAttributeMaxDynamicSharedMemorySize, int(HPipe<S>::bytes())),
+           "cudaFuncSetAttribute");
+    }
     if (pipe_) {
         const int smem = int(EPipe<S>::bytes());
         for (bool sh : {false, true})
@@ -1266,6 +1227,7 @@ Solver<S, T>::Solver(const fdtd_setup_v1& s, int dev, const ShardSpec* shard, bo
                 throw Failure(FDTD_ERR_INVALID, "probe outside the grid or bad component");
             pd[q].off = (long long)((size_t(p.k) * NyT_ + p.j) * NxP_ + p.i);
             pd[q].comp = p.component;
+            probes_E_ = probes_E_ && (p.component <= FDTD_EZ || p.component == FDTD_E_MAG);
         }
         d_probes_ = upload(pd);
         if (nf_) {
@@ -1818,7 +1780,7 @@ void Solver<S, T>::run(uint64_t n) {
     const dim3 blk(32, kBlockY);
     ESrc src{};
     src_static(src);
-    const int pthreads = int(nprobes_ * std::max<uint32_t>(nf_, 1));
+    bool probe_due = false;
     const bool per_kernel = timing_ == FDTD_TIMING_KERNELS;
     const bool fused = n > 0 && begin_fused();
     struct Other {  // the workspace goes back whichever way the run ends
@@ -1844,7 +1806,12 @@ void Solver<S, T>::run(uint64_t n) {
             step_fused(src, int((s - n0) & 1));
             other.n = s + 1 - n0;
         } else {
-            h_kernel()<<<gridH_, blk, hpipe_ ? HPipe<S>::bytes() : 0, st_>>>(a_, kchunkH_, geom_, src.step);
+            const size_t hmem = hpipe_ ? HPipe<S>::bytes() : 0;
+            if (probe_due)
+                h_probe_kernel()<<<dim3(gridH_.x, gridH_.y, gridH_.z + 1), blk, hmem, st_>>>(a_, kchunkH_, geom_, src.step,
+                                                                                            probe_step(s - 1));
+            else h_kernel()<<<gridH_, blk, hmem, st_>>>(a_, kchunkH_, geom_, src.step);
+            probe_due = false;
             if (per_kernel) ck(cudaEventRecord(ev_[1], st_), "cudaEventRecord");
             const size_t smem = pipe_ ? EPipe<S>::bytes() : 0;
             e_kernel(src.ns != 0)<<<gridE_, blk, smem, st_>>>(a_, kchunkE_, src, geom_);
@@ -1853,17 +1820,18 @@ void Solver<S, T>::run(uint64_t n) {
         if (pec_) pec_faces();
         if (per_kernel) ck(cudaEventRecord(ev_[2], st_), "cudaEventRecord");
         if (nprobes_) {
-            const long long sample = (s % save_every_ == 0) ? (long long)(s / save_every_) : -1;
-            k_probe_dft<S, T><<<(pthreads + 127) / 128, 128, 0, st_>>>(a_, d_probes_, int(nprobes_), d_freqs_, int(nf_),
-                                                                         d_dft_, d_series_, sample, double(s + 1) * dt_, dt_,
-                                                                         sE_, sH_);
-            ++launches;
-            if (sample >= 0) series_count_ = uint64_t(sample) + 1;
+            // E does not change until the next E sweep: on a small grid, probes that read only E ride
+            // along with the next step's H sweep instead of taking a launch of their own (us per step:
+            // 48^3 21.7 -> 18, 80^3 25.2 -> 22, 157x121x93 46.5 -> 44.6, 173x131x97 FP64 122.8 -> 122;
+            // above 2.5 M cells the launch is under 4 % of a step and is not seen)
+            probe_due = path_ == 1 && !fused && !per_kernel && probes_E_ && s + 1 < last && nflat_ <= 2500000;
+            if (!probe_due) launch_probes(s);
+            if (s % save_every_ == 0) series_count_ = s / save_every_ + 1;
         }
         if (writer_ && !oplan_.movies.empty() && s % save_every_ == 0) capture_movies();
         if (writer_ && oplan_.tls && s % save_every_ == 0) capture_tls(s);
         if (interval_ && s % interval_ == 0) {
-            k_monitor_reduce<S, T><<<8 * 148, 256, 0, st_>>>(a_, size_t(shard_.own0) * plane_, size_t(shard_.own1) * plane_,
+            k_monitor_reduce<S, T><<<mon_blocks(), 256, 0, st_>>>(a_, size_t(shard_.own0) * plane_, size_t(shard_.own1) * plane_,
                                                              d_dx_, d_dy_, d_dz_, int((s + 1) & 1), d_acc_, sE_);
             k_monitor_eval<<<1, 1, 0, st_>>>(d_acc_, d_ms_, d_status_, s);
             launches += 2;
@@ -1924,16 +1892,11 @@ void Solver<S, T>::phase_E(uint64_t s, ESrc& src, bool monitor) {
     ++launches;
     if (pec_) pec_faces();
     if (nprobes_) {
-        const int pthreads = int(nprobes_ * std::max<uint32_t>(nf_, 1));
-        const long long sample = (s % save_every_ == 0) ? (long long)(s / save_every_) : -1;
-        k_probe_dft<S, T><<<(pthreads + 127) / 128, 128, 0, st_>>>(a_, d_probes_, int(nprobes_), d_freqs_, int(nf_),
-                                                                     d_dft_, d_series_, sample, double(s + 1) * dt_, dt_,
-                                                                     sE_, sH_);
-        ++launches;
-        if (sample >= 0) series_count_ = uint64_t(sample) + 1;
+        launch_probes(s);
+        if (s % save_every_ == 0) series_count_ = s / save_every_ + 1;
     }
     if (monitor) {
-        k_monitor_reduce<S, T><<<8 * 148, 256, 0, st_>>>(a_, size_t(shard_.own0) * plane_, size_t(shard_.own1) * plane_,
+        k_monitor_reduce<S, T><<<mon_blocks(), 256, 0, st_>>>(a_, size_t(shard_.own0) * plane_, size_t(shard_.own1) * plane_,
                                                          d_dx_, d_dy_, d_dz_, int((s + 1) & 1), d_acc_, sE_);
         ++launches;
     }
