@@ -634,12 +634,13 @@ DTYPE = {"fp32": "f32", "fp64": "f64", "fp16": "f32 (fp16 storage)", "bf16": "f3
 
 def shards_for(args, form: str) -> int:
     """z shards of the solve on the GPU for a storage form: --shards, else the fastest measured
-    on the 536^3 workload (one B200, 20 x 10 steps): FP64 steps fastest whole (37.0 against 36.7
-    with 2 shards and 36.5 with 4); FP32, BF16 and FP16 with 4 shards (72.6 / 101.8 / 104.6
-    against 72.2 / 97.5 / 100.8 whole), whose sweeps' tails overlap on their streams."""
+    on the 536^3 workload (one B200): FP64 and FP32 step fastest whole, with one launch per step
+    (45 and 80 Gcell-updates/s; 36.5 and 72.6 as 4 shards, which take two sweeps); BF16 and FP16
+    with 4 shards (101.8 / 104.6 against 97.5 / 100.8 whole, in an earlier build), whose sweeps'
+    tails overlap on their streams."""
     if args.shards:
         return args.shards
-    return 1 if form == "fp64" else 4
+    return 1 if form in ("fp64", "fp32") else 4
 
 
 def workload_config(setup, cfg: str, desc: str) -> dict:
