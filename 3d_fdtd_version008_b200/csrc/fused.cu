@@ -25,14 +25,24 @@ __device__ __forceinline__ bool mbar_try(uint64_t* b, unsigned parity) {
         : "memory");
     return ok != 0;
 }
-// Bounded wait for a phase: false when kMaxTries attempts (each suspends the warp for up to 2 us;
-// seconds in all) have failed.
-constexpr int kMaxTries = 1 << 21;
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned parity) {
-    for (int n = 0; n < kMaxTries; ++n)
+__device__ __forceinline__ unsigned ns_now() {
+    unsigned t;
+    asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
+    return t;
+}
+// Bounded wait for a phase: false when `limit` ns (below 2^31) have passed, or when another wait of
+// the block has failed (what this one waits for may then never come).
+__device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned parity, unsigned limit, volatile unsigned* failed) {
+    if (mbar_try(b, parity)) return true;
+    const unsigned t0 = ns_now();
+    do {
         if (mbar_try(b, parity)) return true;
+    } while (*failed == 0u && ns_now() - t0 < limit);
+    *failed = 1u;
     return false;
 }
+constexpr unsigned kDrainNs = 1000000000u;  // bound on waiting for copies in flight before a block gives up
+
 __device__ __forceinline__ void tma_load4(void* dst, const CUtensorMap* m, int x, int y, int z, int c, uint64_t* bar) {
     asm volatile(
         "cp.async.bulk.tensor.4d.shared::cta.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
@@ -40,10 +50,6 @@ __device__ __forceinline__ void tma_load4(void* dst, const CUtensorMap* m, int x
         "l"(m), "r"(x), "r"(y), "r"(z), "r"(c), "r"(unsigned(__cvta_generic_to_shared(bar)))
         : "memory");
 }
-
-// Keeps a value in its register: the compiler may not load it again where it is used.
-__device__ __forceinline__ void opaque(float& v) { asm volatile("" : "+f"(v)); }
-__device__ __forceinline__ void opaque(double& v) { asm volatile("" : "+d"(v)); }
 
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
@@ -152,6 +158,8 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
     // full: the stage's copies have arrived; freed: every warp has read it for the last time;
     // xfull: the row's new Hx and Hz are in the stage
     __shared__ uint64_t full[NS], freed[NS], xfull[NS][TY];
+    __shared__ unsigned failed;  // a wait of this block has run out
+    __shared__ int issued;       // the last ring position whose copies were asked for
     int lane, w;  // opaque, so that they stay in registers
     asm volatile("mov.u32 %0, %%tid.x;" : "=r"(lane));
     asm volatile("mov.u32 %0, %%tid.y;" : "=r"(w));
@@ -175,8 +183,9 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
         for (int s = 0; s < NS; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&freed[s], TY + 1);
-            for (int r = 0; r < TY; ++r) mbar_init(&xfull[s][r], 1);
+            for (int r = 0; r < TY; ++r) mbar_init(&xfull[s][r], 1 + g.hold);
         }
+        failed = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         // the first planes' copies, unless a failed monitor step has stopped the solve (one thread
@@ -188,6 +197,7 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
 #pragma unroll
             for (int p = 1; p < NS; ++p)
                 if (k0 + p - 1 < ke) issue(k0 + p - 1, p);
+            issued = min(NS - 1, ke - k0);
         }
     }
     // The tile's coefficients, so that a plane waits for no global load of them: along x (1/dx and,
@@ -268,7 +278,8 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
     unsigned xq = unsigned(xpsi_at(a, k0, row_in ? j : 0, x0));  // the vector's x-slab psi, y-slab psi
     unsigned yq = unsigned(k0 * np2 + jy) * unsigned(a.NxP) + unsigned(x0);
     unsigned xstep = unsigned(a.NyT) * unsigned(XSlab(a.NxT, np, W).len), ystep = unsigned(np2) * unsigned(a.NxP);
-    bool ok = mbar_wait(&full[0], 0);
+    auto wait = [&](uint64_t* b, unsigned parity) { return mbar_wait(b, parity, g.wait_ns, &failed); };
+    bool ok = wait(&full[0], 0);
 
     // G: with everything a plane may need; else the plain update.
     auto plane = [&](auto general, const int k) __attribute__((always_inline)) {
@@ -286,7 +297,7 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
         T ex[W], ey[W], ez[W], hx[W], hy[W], hz[W];
         T px0[W], px1[W];  // x-slab psi, issued before the wait
         if (G && xpml && hup) { Vec<T>::ld(old.p[3] + xq, px0); Vec<T>::ld(old.p[4] + xq, px1); }
-        ok = ok && mbar_wait(&full[sc], ph);
+        ok = ok && wait(&full[sc], ph);
         T* const ecur = stage(sc) + wv * XW + lanev;
         Vec<T>::ld(eprev, ex);
         Vec<T>::ld(eprev + EC, ey);
@@ -348,14 +359,15 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
         if (w == 0) {
             // E(k) is read: its stage takes the next plane
             if (k + NS - 1 < ke) {
-                ok = ok && mbar_wait(&freed[sp], php);
+                ok = ok && wait(&freed[sp], php);
                 if (leader && ok) {
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // H was written into the stage
                     issue(k + NS - 1, sp);
+                    issued = k + NS - k0;
                 }
             }
         } else if (k >= kb) {
-            ok = ok && mbar_wait(&xfull[sc][w - 1], ph);
+            ok = ok && wait(&xfull[sc][w - 1], ph);
         }
 
         if (eup) {  // uniform in the warp
@@ -410,7 +422,7 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
         for (int e = 0; e < W; ++e) { hxm[e] = hx[e]; hym[e] = hy[e]; }
         eprev = ecur;
     };
-    for (int k = k0; k < ke && ok; ++k) {
+    for (int k = k0; k < ke; ++k) {  // to the end after a failed wait too: a plane's shuffles take every lane
         const bool gen = gen_col || in_pml(k + a.kz0, a.NzG, np) || k + a.kz0 >= a.NzG - 1 || k + a.kz0 < 1 ||
                          (gain_col && k >= a.gk0 && k < a.gk0 + a.gZ);
         if (gen) plane(std::true_type{}, k);
@@ -429,7 +441,14 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
         php = ph;
         if (++sc == NS) { sc = 0; ph ^= 1u; }
     }
-    if (!ok) atomicOr(status_w, kStatusTimeout);  // a wait ran out: flag it and leave
+    if (!ok) {  // a wait ran out: flag it and leave
+        atomicOr(status_w, kStatusTimeout);
+        if (leader) {  // ... but not before the copies in flight, whose target is the block's shared memory
+            const unsigned t0 = ns_now();
+            for (int m = max(issued - NS + 1, 0); m <= issued; ++m)
+                while (!mbar_try(&full[m % NS], unsigned(m / NS) & 1u) && ns_now() - t0 < kDrainNs) {}
+        }
+    }
 }
 
 template <typename T>

@@ -46,6 +46,8 @@ struct FusedGeom {
     int gx, gy;  // tiles in x, in y
     int kc;      // planes per chunk
     int nrow;    // material rows
+    unsigned wait_ns;  // bound on one wait in the kernel, below 2^31
+    int hold;    // 1: the row-ready barriers never complete, so that the waits on them run out
 };
 
 template <typename T>

@@ -1297,6 +1297,13 @@ Solver<S, T>::Solver(const fdtd_setup_v1& s, int dev, const ShardSpec* shard, bo
     ck(cudaStreamSynchronize(st_), "setup upload");
 }
 
+// Bound on one wait of a kernel that waits (the slab-ordered and the fused step): FDTD_B200_WAIT_NS
+// nanoseconds (at least 1000), else 2 s.
+unsigned long long wait_limit_ns() {
+    if (const char* e = std::getenv("FDTD_B200_WAIT_NS")) return std::max(1000ull, std::strtoull(e, nullptr, 10));
+    return kWaitNs;
+}
+
 // The fused step's tiles and chunks, and whether the solve takes it.
 template <typename S, typename T>
 void Solver<S, T>::setup_fused() {
@@ -1304,6 +1311,10 @@ void Solver<S, T>::setup_fused() {
     constexpr int W = F::W;
     FusedGeom& f = fgeom_;
     f.nrow = int(mat_rows_);
+    f.wait_ns = unsigned(std::min<unsigned long long>(wait_limit_ns(), 0x7fffffffull));
+    // FDTD_B200_FUSED_HOLD=1: the waits for the row below run out (how the bounded wait is tested)
+    f.hold = 0;
+    if (const char* e = std::getenv("FDTD_B200_FUSED_HOLD")) f.hold = std::string(e) == "1";
     const int nv = (NxT_ + W - 1) / W;
     f.gx = (nv + F::kMaxU - 1) / F::kMaxU;
     f.u = int(round_up(size_t((nv + f.gx - 1) / f.gx), F::kAlignU));
@@ -1474,11 +1485,9 @@ void Solver<S, T>::setup_slabs() {
     plan_.gxE = int(gridE_.x);
     plan_.nE = int(gridE_.x * gridE_.y);
     if ((long long)plan_.nslab * (plan_.nH + plan_.nE) > 0x7fffffffLL) throw Failure(FDTD_ERR_INVALID, "grid too large for the slab-ordered step");
-    // Bound on one dependency wait of an E tile: FDTD_B200_WAIT_NS nanoseconds (at least 1000),
-    // else 2 s.  FDTD_B200_SLAB_HOLD=1 leaves the hold word set, so that every E tile's wait
-    // runs out and the step ends with FDTD_ERR_TIMEOUT (how the bounded wait is tested).
-    plan_.wait_ns = kWaitNs;
-    if (const char* e = std::getenv("FDTD_B200_WAIT_NS")) plan_.wait_ns = std::max(1000ull, std::strtoull(e, nullptr, 10));
+    // FDTD_B200_SLAB_HOLD=1 leaves the hold word set, so that every E tile's wait runs out and
+    // the step ends with FDTD_ERR_TIMEOUT (how the bounded wait is tested).
+    plan_.wait_ns = wait_limit_ns();
     if (const char* e = std::getenv("FDTD_B200_SLAB_HOLD")) slab_hold_ = std::string(e) == "1";
     d_ctr_ = alloc<unsigned>(size_t(plan_.nslab) + 2);
     int sms = 148, per = 0;
