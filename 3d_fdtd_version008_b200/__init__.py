@@ -49,7 +49,7 @@ EXPORTED_SYMBOLS = (
     "fdtd_set_tls_state", "fdtd_get_tls_state", "fdtd_run", "fdtd_steps_done",
     "fdtd_get_probe_series", "fdtd_get_dft", "fdtd_get_diagnostics", "fdtd_device_bytes",
     "fdtd_kernel_launches", "fdtd_set_timing", "fdtd_get_timing", "fdtd_set_kernel_path", "fdtd_synchronize", "fdtd_last_error",
-    "fdtd_destroy", "fdtd_field_scan_noalloc", "fdtd_attach_outputs", "fdtd_flush_outputs", "fdtd_material_rows",
+    "fdtd_destroy", "fdtd_field_scan_noalloc", "fdtd_attach_outputs", "fdtd_flush_outputs", "fdtd_material_rows", "fdtd_fused_planes",
     "fdtd_create_sharded",
     "fdtd_close_outputs",
     "fdtd_batch_create", "fdtd_batch_submit", "fdtd_batch_run", "fdtd_batch_job_state",
@@ -161,6 +161,7 @@ def load_library() -> C.CDLL:
         "fdtd_attach_outputs": (C.c_int, [vp, vp, C.c_char_p]),
         "fdtd_flush_outputs": (C.c_int, [vp]),
         "fdtd_material_rows": (C.c_int, [vp, C.POINTER(C.c_uint64)]),
+        "fdtd_fused_planes": (C.c_int, [vp, C.POINTER(C.c_uint64)]),
         "fdtd_create_sharded": (C.c_int, [C.POINTER(SetupV1), C.c_int, C.POINTER(C.c_int), C.POINTER(vp)]),
         "fdtd_close_outputs": (C.c_int, [vp]),
         "fdtd_create": (C.c_int, [C.POINTER(SetupV1), C.c_int, C.POINTER(vp)]),
@@ -366,6 +367,13 @@ class Solver:
         """Distinct bE rows when the material is held as a row index per cell, else 0."""
         n = C.c_uint64()
         self._check(load_library().fdtd_material_rows(self._h, C.byref(n)), "fdtd_material_rows")
+        return n.value
+
+    @property
+    def fused_planes(self) -> int:
+        """z planes per block of the one-launch step that run() takes, or 0: two sweeps."""
+        n = C.c_uint64()
+        self._check(load_library().fdtd_fused_planes(self._h, C.byref(n)), "fdtd_fused_planes")
         return n.value
 
     @property

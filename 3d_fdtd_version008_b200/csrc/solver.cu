@@ -577,7 +577,7 @@ public:
     virtual void attach_outputs(const fdtd::SimSetup& setup, const std::string& root) = 0;
     virtual void flush_outputs() = 0;
     virtual void close_outputs() = 0;
-    uint64_t steps = 0, launches = 0, dev_bytes = 0, material_rows = 0;
+    uint64_t steps = 0, launches = 0, dev_bytes = 0, material_rows = 0, fused_planes = 0;
     int device = 0;
 };
 
@@ -1329,6 +1329,7 @@ void Solver<S, T>::setup_fused() {
         const double cost = nb <= slots ? kc + 3 : nb / slots * (kc + 3) + 0.5 * (kc + 3);
         if (cost < best) { best = cost; f.kc = kc; }
     }
+    if (const char* e = std::getenv("FDTD_B200_FUSED_KCHUNK")) f.kc = std::clamp(std::atoi(e), 1, std::min(NzT_, int(F::kMaxKc)));
     // Which solves: a tile row takes a warp whatever it owns, so a row's vectors must fill most of
     // its tiles (four fifths of 30 each); and a CPML slab costs the fused step more (its psi is
     // loaded within a warp's plane, and one x-slab vector slows its whole row segment), so that
@@ -1348,6 +1349,7 @@ void Solver<S, T>::setup_fused() {
     fusable_ = take && a_.bidx != nullptr && std::max({xs, ys, zs, plane_}) < (size_t(1) << 31) && f.gy <= 65535 &&
                (NzT_ + f.kc - 1) / f.kc <= 65535;
     if (!fusable_) return;
+    fused_planes = uint64_t(f.kc);
     for (bool sh : {false, true})
         ck(cudaFuncSetAttribute(fused_kernel<T>(sh), cudaFuncAttributeMaxDynamicSharedMemorySize, int(F::bytes())),
            "cudaFuncSetAttribute");
@@ -3699,6 +3701,7 @@ int fdtd_get_diagnostics(fdtd_handle* h, fdtd_diagnostics_v1* d) { if (!h || !d)
 int fdtd_device_bytes(const fdtd_handle* h, uint64_t* b) { if (!h || !b) return FDTD_ERR_INVALID; *b = h->s->dev_bytes; return FDTD_OK; }
 int fdtd_kernel_launches(const fdtd_handle* h, uint64_t* n) { if (!h || !n) return FDTD_ERR_INVALID; *n = h->s->launches; return FDTD_OK; }
 int fdtd_material_rows(const fdtd_handle* h, uint64_t* rows) { if (!h || !rows) return FDTD_ERR_INVALID; *rows = h->s->material_rows; return FDTD_OK; }
+int fdtd_fused_planes(const fdtd_handle* h, uint64_t* planes) { if (!h || !planes) return FDTD_ERR_INVALID; *planes = h->s->fused_planes; return FDTD_OK; }
 int fdtd_set_timing(fdtd_handle* h, int mode) { if (!h) return FDTD_ERR_INVALID; return guarded(h, [&] { h->s->set_timing(mode); }); }
 int fdtd_get_timing(fdtd_handle* h, fdtd_timing_v1* t) { if (!h || !t) return FDTD_ERR_INVALID; return guarded(h, [&] { h->s->timing(t); }); }
 int fdtd_set_kernel_path(fdtd_handle* h, int path) { if (!h) return FDTD_ERR_INVALID; return guarded(h, [&] { h->s->set_path(path); }); }

@@ -267,6 +267,8 @@ int fdtd_kernel_launches(const fdtd_handle *h, uint64_t *n);
  * 2-byte row index per cell and a table of the rows (at most 65535 rows), 0 when it keeps the
  * three arrays.  Results are the same either way. */
 int fdtd_material_rows(const fdtd_handle *h, uint64_t *rows);
+/* z planes per block of the one-launch step that the handle's runs take, or 0: two sweeps. */
+int fdtd_fused_planes(const fdtd_handle *h, uint64_t *planes);
 /* Select FDTD_TIMING_OFF / _RUN / _KERNELS; any call resets the totals. */
 int fdtd_set_timing(fdtd_handle *h, int mode);
 int fdtd_get_timing(fdtd_handle *h, fdtd_timing_v1 *out);
