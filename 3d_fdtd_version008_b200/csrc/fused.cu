@@ -373,7 +373,7 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
         if (eup) {  // uniform in the warp
             const T* const xs = ecur + 3 * EC - XW;  // the row below
             const T hzp = __shfl_up_sync(kFull, hz[W - 1], 1), hyp = __shfl_up_sync(kFull, hy[W - 1], 1);
-            const bool special = G && srow && src_in_vector<SH>(src, x0, j, k, W);
+            const unsigned special = G && srow ? src_in_vector<SH>(src, x0, j, k, W) : 0u;
             T bx[W], by[W], bz[W];
             rows_of(smat, a.btab, ids, bx, by, bz);
             T t[W], da[W], db[W], idx[W];
@@ -385,7 +385,7 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
             if (G && ypml) psi_yz(da, a.psiE[0], a.psiE[0], yq, ys1, own, own, yc + 3, yc[5], a.psc);
             if (G && zpml) psi_yz(db, a.psiE[1], a.psiE[1], zq, zs, own, own, zc + 3, zc[5], a.psc);
             vsub(da, db);
-            if (G && special) sub_J<SH>(src, 0, x0, j, k, da);
+            if (G && special) sub_J<SH>(src, special, 0, x0, j, k, da);
             update<G>(ex, bx, da, me);
             // Ey: dHx/dz - dHz/dx
             vdq(da, hx, hxm, idz);
@@ -395,7 +395,7 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
             if (G && zpml) psi_yz(da, a.psiE[2], a.psiE[2], zq, zs, own, own, zc + 3, zc[5], a.psc);
             if (G && xgen) psi_x(db, px0, a.psiE[3], a.psiE[3], xq, xs1, xpml && own, xco + 3 * XW, xco + 4 * XW, xco + 5 * XW, mx, a.psc);
             vsub(da, db);
-            if (G && special) sub_J<SH>(src, 1, x0, j, k, da);
+            if (G && special) sub_J<SH>(src, special, 1, x0, j, k, da);
             update<G>(ey, by, da, me);
             // Ez: dHy/dx - dHx/dy
             Vec<T>::ld(xs, t);
@@ -406,7 +406,7 @@ k_step_fused(const __grid_constant__ CUtensorMap mapE, const __grid_constant__ C
             if (G && xgen) psi_x(da, px1, a.psiE[4], a.psiE[4], xq, xs1, xpml && own, xco + 3 * XW, xco + 4 * XW, xco + 5 * XW, mx, a.psc);
             if (G && ypml) psi_yz(db, a.psiE[5], a.psiE[5], yq, ys1, own, own, yc + 3, yc[5], a.psc);
             vsub(da, db);
-            if (G && special) sub_J<SH>(src, 2, x0, j, k, da);
+            if (G && special) sub_J<SH>(src, special, 2, x0, j, k, da);
             if (G && grow && k >= a.gk0 && k < a.gk0 + a.gZ) {
                 gain_vector(a, src.parity, x0, j, k, me, da, bz, ez);
             } else {

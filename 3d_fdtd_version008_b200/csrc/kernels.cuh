@@ -560,59 +560,56 @@ struct EPipe : PipeShape<sizeof(S) == 2 ? 8 : 16, sizeof(S) == 2 ? 4 : 2> {
     static constexpr size_t bytes() { return size_t(EPipe::kStages) * kSlots * (32 * kBlockY) * EPipe::SB; }
 };
 
-// True when a point source or (SH) a plane-wave sheet touches one of the W cells (i0.., j, k).
+// Non-zero when a point source or (SH) a plane-wave sheet touches one of the W cells (i0.., j, k).
+// With sheets, bit s for point source s and bit kMaxSources + s for sheet s.
 template <bool SH>
-__device__ __forceinline__ bool src_in_vector(const ESrc& src, int i0, int j, int k, int W) {
-    bool hit = false;
+__device__ __forceinline__ unsigned src_in_vector(const ESrc& src, int i0, int j, int k, int W) {
+    unsigned hit = 0;
     for (int s = 0; s < src.n; ++s)
-        hit |= src.sj[s] == j && src.sk[s] == k && src.si[s] >= i0 && src.si[s] < i0 + W;
+        hit |= unsigned(src.sj[s] == j && src.sk[s] == k && src.si[s] >= i0 && src.si[s] < i0 + W) << (SH ? s : 0);
     if constexpr (SH) for (int s = 0; s < src.ns; ++s) {
+        bool in;
         if (src.ax[s] == 2)
-            hit |= k == src.pl[s] && j >= src.lo1[s] && j <= src.hi1[s] && i0 + W > src.lo0[s] && i0 <= src.hi0[s];
+            in = k == src.pl[s] && j >= src.lo1[s] && j <= src.hi1[s] && i0 + W > src.lo0[s] && i0 <= src.hi0[s];
         else if (src.ax[s] == 1)
-            hit |= j == src.pl[s] && k >= src.lo1[s] && k <= src.hi1[s] && i0 + W > src.lo0[s] && i0 <= src.hi0[s];
+            in = j == src.pl[s] && k >= src.lo1[s] && k <= src.hi1[s] && i0 + W > src.lo0[s] && i0 <= src.hi0[s];
         else
-            hit |= src.pl[s] >= i0 && src.pl[s] < i0 + W && j >= src.lo0[s] && j <= src.hi0[s] && k >= src.lo1[s] &&
-                   k <= src.hi1[s];
+            in = src.pl[s] >= i0 && src.pl[s] < i0 + W && j >= src.lo0[s] && j <= src.hi0[s] && k >= src.lo1[s] &&
+                 k <= src.hi1[s];
+        hit |= unsigned(in) << (kMaxSources + s);
     }
     return hit;
 }
 
-// J of the plane-wave sheets at cell (i, j, k), added after the point sources (the
-// reference's source registration order).
-template <typename T>
-__device__ __forceinline__ void sheet_J(const ESrc& src, int i, int j, int k, T& Jx, T& Jy, T& Jz) {
-    for (int s = 0; s < src.ns; ++s) {
-        bool in;
-        if (src.ax[s] == 2) in = k == src.pl[s] && i >= src.lo0[s] && i <= src.hi0[s] && j >= src.lo1[s] && j <= src.hi1[s];
-        else if (src.ax[s] == 1) in = j == src.pl[s] && i >= src.lo0[s] && i <= src.hi0[s] && k >= src.lo1[s] && k <= src.hi1[s];
-        else in = i == src.pl[s] && j >= src.lo0[s] && j <= src.hi0[s] && k >= src.lo1[s] && k <= src.hi1[s];
-        if (in) {
-            const T v = T(src.sJ[s]);
-            if (src.pc[s] == 0) Jx = add_rn(Jx, v);
-            else if (src.pc[s] == 1) Jy = add_rn(Jy, v);
-            else Jz = add_rn(Jz, v);
-        }
-    }
-}
-
-// Current of the step's sources into component comp at cell (i, j, k): the point sources, then the sheets.
-template <bool SH, typename T>
-__device__ __forceinline__ T source_J(const ESrc& src, int comp, int i, int j, int k) {
-    T J = 0;
-    for (int s = 0; s < src.n; ++s)
-        if (src.sc[s] == comp && src.si[s] == i && src.sj[s] == j && src.sk[s] == k) J = add_rn(J, T(src.J[s]));
-    if constexpr (SH) {
-        T Jx = comp == 0 ? J : T(0), Jy = comp == 1 ? J : T(0), Jz = comp == 2 ? J : T(0);
-        sheet_J(src, i, j, k, Jx, Jy, Jz);
-        J = comp == 0 ? Jx : comp == 1 ? Jy : Jz;
-    }
-    return J;
-}
-template <bool SH, typename T>
-__device__ __forceinline__ void sub_J(const ESrc& src, int comp, int x0, int j, int k, T (&c)[Vec<T>::W]) {
+// Subtracts the current of the step's sources into component comp from that component's curl in a
+// vector that src_in_vector found touched (hit): J sums the point sources, then the sheets (the
+// reference's source registration order).  With sheets only the sources in `hit` are looked at, as a
+// sheet normal to x puts a vector of every row here: testing them all for each cell and component
+// took 617 us per step on 280^3 FP32 with a sheet normal to z and one to x, this takes 399 (BF16 595
+// -> 355, FP64 804 -> 675).  Without, the few vectors of the point sources test them all, which
+// holds no mask over the update (it spilled).
+template <bool SH, typename T, int W>
+__device__ __forceinline__ void sub_J(const ESrc& src, unsigned hit, int comp, int x0, int j, int k, T (&c)[W]) {
 #pragma unroll
-    for (int e = 0; e < Vec<T>::W; ++e) c[e] = sub_rn(c[e], source_J<SH, T>(src, comp, x0 + e, j, k));
+    for (int e = 0; e < W; ++e) {
+        T J = T(0);
+        if constexpr (SH) {
+            for (unsigned m = hit; m != 0u; m &= m - 1u) {
+                const int s = __ffs(int(m)) - 1;
+                if (s < kMaxSources) {
+                    if (src.sc[s] == comp && src.si[s] == x0 + e) J = add_rn(J, T(src.J[s]));
+                } else {
+                    const int q = s - kMaxSources;
+                    const int lo = src.ax[q] == 0 ? src.pl[q] : src.lo0[q], hi = src.ax[q] == 0 ? src.pl[q] : src.hi0[q];
+                    if (src.pc[q] == comp && x0 + e >= lo && x0 + e <= hi) J = add_rn(J, T(src.sJ[q]));
+                }
+            }
+        } else {
+            for (int s = 0; s < src.n; ++s)
+                if (src.sc[s] == comp && src.si[s] == x0 + e && src.sj[s] == j && src.sk[s] == k) J = add_rn(J, T(src.J[s]));
+        }
+        c[e] = sub_rn(c[e], J);
+    }
 }
 
 // Two-level gain of one vector in plane k: polarization with E^n, Ez += bz (curl - dP/dt), populations with
@@ -1455,7 +1452,7 @@ __device__ __forceinline__ void e_column(const StepArgs<S, T>& a, const SweepGeo
             continue;
         }
         // (as in h_column; the x = 0 plane and the padding are never updated)
-        const bool special = act && src_in_vector<SH>(src, i0, j, k, W);
+        const unsigned special = act ? src_in_vector<SH>(src, i0, j, k, W) : 0u;
         T da[W], db[W], xb[W], xc[W], xk[W];
         if (xpml) { Vec<T>::ldg(a.pbE[0] + i0, xb); Vec<T>::ldg(a.pcE[0] + i0, xc); Vec<T>::ldg(a.ik[0] + i0, xk); }
         vdq(da, hz, hzj, idy);  // dHz/dy
@@ -1463,7 +1460,7 @@ __device__ __forceinline__ void e_column(const StepArgs<S, T>& a, const SweepGeo
         if (ypml) pml_yz<S>(da, yb, yc, yik, pxy, a.psc);
         if (zpml) pml_yz<S>(db, zb, zc, zik, pxz, a.psc);
         vsub(da, db);
-        if (special) sub_J<SH>(src, 0, i0, j, k, da);
+        if (special) sub_J<SH>(src, special, 0, i0, j, k, da);
         vfma_in(ex, bx, da, mask.e);
         vdq(da, hx, hxm, idz);  // dHx/dz
 #pragma unroll
@@ -1472,7 +1469,7 @@ __device__ __forceinline__ void e_column(const StepArgs<S, T>& a, const SweepGeo
         if (zpml) pml_yz<S>(da, zb, zc, zik, pyz, a.psc);
         if (xpml) pml_x<S>(db, xb, xc, xk, mask.x, x3, a.psc);
         vsub(da, db);
-        if (special) sub_J<SH>(src, 1, i0, j, k, da);
+        if (special) sub_J<SH>(src, special, 1, i0, j, k, da);
         vfma_in(ey, by, da, mask.e);
 #pragma unroll
         for (int e = 0; e < W; ++e) da[e] = sub_rn(hy[e], (e > 0) ? hy[e - 1] : hyp);
@@ -1481,7 +1478,7 @@ __device__ __forceinline__ void e_column(const StepArgs<S, T>& a, const SweepGeo
         if (xpml) pml_x<S>(da, xb, xc, xk, mask.x, x4, a.psc);
         if (ypml) pml_yz<S>(db, yb, yc, yik, pzy, a.psc);
         vsub(da, db);
-        if (special) sub_J<SH>(src, 2, i0, j, k, da);
+        if (special) sub_J<SH>(src, special, 2, i0, j, k, da);
         if (gplane) gain_vector(a, src.parity, i0, j, k, mask.e, da, bz, ez);
         else vfma_in(ez, bz, da, mask.e);
         if (act) {
