@@ -5,7 +5,7 @@
 // memory twice.  Here a step reads the fields from one copy and writes them to another: a block
 // can then recompute the H it needs of its neighbours' cells (the row below, the column to the
 // left, the plane below) from values nobody overwrites, and E and H are read once and written
-// once per step.  The second copy is a workspace of the running call.
+// once per step.  The second copy is shared by the handles of a device (IdleCopies in solver.cu).
 //
 // A block owns TY rows of a tile of u vectors in x and marches in +z through a chunk of planes.
 // Warp w holds row j0 - 1 + w: warp 0 the row below the tile (H only), warps 1 .. TY the owned

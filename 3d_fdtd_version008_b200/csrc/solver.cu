@@ -559,6 +559,113 @@ struct ShardSpec {
     double psi_dx = 0;  // 16-bit storage: the whole solve's smallest cell edge (0: this grid's)
 };
 
+// The second copies of the fields that fused steps write to (Solver::run), of one device: a run takes
+// one and gives it back, to this handle's next run or another's of the same size.  Taken from and
+// returned to the memory pool in each run, as it first was, a copy now and then cost tens to hundreds of
+// ms in a process with several solves, when the pool moved its memory about (320^3 FP32, 100 steps:
+// 64 ms on the device, up to 136 by the clock).  Idle copies: at most kIdle and an eighth of the
+// device's memory (the oldest go first); all return to the pool when the last handle that may use one
+// is destroyed, or when a solve's own allocation fails (Solver::dev_alloc).
+class IdleCopies {
+public:
+    static IdleCopies& of(int dev) {
+        static std::mutex m;
+        static std::map<int, IdleCopies*> all;  // never freed: released with the process
+        std::lock_guard<std::mutex> l(m);
+        IdleCopies*& q = all[dev];
+        if (!q) q = new IdleCopies(dev);
+        return *q;
+    }
+    // null: there is none of that size
+    void* take(size_t bytes) {
+        std::lock_guard<std::mutex> l(mu_);
+        for (size_t q = 0; q < idle_.size(); ++q)
+            if (idle_[q].bytes == bytes) {
+                void* const p = idle_[q].p;
+                held_ -= bytes;
+                idle_.erase(idle_.begin() + q);
+                return p;
+            }
+        return nullptr;
+    }
+    // no work on the copy may be pending
+    void put(void* p, size_t bytes) {
+        std::vector<Buf> out;
+        {
+            std::lock_guard<std::mutex> l(mu_);
+            idle_.push_back(Buf{p, bytes});
+            held_ += bytes;
+            while (!idle_.empty() && (idle_.size() > kIdle || held_ > limit_)) {
+                out.push_back(idle_.front());
+                held_ -= idle_.front().bytes;
+                idle_.erase(idle_.begin());
+            }
+        }
+        release(out);
+    }
+    // returns all idle copies to the pool; false: there were none
+    bool flush() {
+        std::vector<Buf> out;
+        {
+            std::lock_guard<std::mutex> l(mu_);
+            out.swap(idle_);
+            held_ = 0;
+        }
+        release(out);
+        return !out.empty();
+    }
+    // A handle that may take copies holds one of these.
+    class User {
+    public:
+        User() = default;
+        User(const User&) = delete;
+        User& operator=(const User&) = delete;
+        ~User() {
+            if (!c_) return;
+            bool last;
+            {
+                std::lock_guard<std::mutex> l(c_->mu_);
+                last = --c_->users_ == 0;
+            }
+            if (last) c_->flush();
+        }
+        void join(int dev) {
+            c_ = &of(dev);
+            std::lock_guard<std::mutex> l(c_->mu_);
+            ++c_->users_;
+        }
+
+    private:
+        IdleCopies* c_ = nullptr;
+    };
+
+private:
+    struct Buf {
+        void* p;
+        size_t bytes;
+    };
+    explicit IdleCopies(int dev) : dev_(dev) {
+        size_t free_b = 0, total = 0;
+        ck(cudaMemGetInfo(&free_b, &total), "cudaMemGetInfo");
+        limit_ = total / 8;
+    }
+    void release(const std::vector<Buf>& out) {
+        if (out.empty()) return;
+        int now = 0;
+        cudaGetDevice(&now);
+        cudaSetDevice(dev_);
+        for (const Buf& b : out) cudaFreeAsync(b.p, cudaStreamPerThread);
+        cudaStreamSynchronize(cudaStreamPerThread);  // now any stream's allocation may have them
+        cudaSetDevice(now);
+    }
+    static constexpr size_t kIdle = 4;
+    const int dev_;
+    size_t limit_ = 0, held_ = 0;
+    int users_ = 0;
+    std::mutex mu_;
+    std::vector<Buf> idle_;
+};
+
 class SolverBase {
 public:
     virtual ~SolverBase() = default;
@@ -641,8 +748,13 @@ private:
     // 7-8 ms through cudaMalloc, and the FP64 sweeps ran 0.7 % slower on cudaMalloc'd fields.
     bool pooled_ = true;
     void dev_alloc(void** p, size_t bytes) {
-        if (pooled_) ck(cudaMallocAsync(p, bytes, st_), "cudaMallocAsync");
-        else ck(cudaMalloc(p, bytes), "cudaMalloc");
+        auto get = [&] { return pooled_ ? cudaMallocAsync(p, bytes, st_) : cudaMalloc(p, bytes); };
+        cudaError_t e = get();
+        if (e == cudaErrorMemoryAllocation && IdleCopies::of(device).flush()) {
+            cudaGetLastError();
+            e = get();
+        }
+        ck(e, pooled_ ? "cudaMallocAsync" : "cudaMalloc");
     }
     void dev_free(void* p) {
         if (pooled_) cudaFreeAsync(p, st_);
@@ -822,6 +934,11 @@ private:
         S* f = nullptr;
         S* psi = nullptr;
     };
+    size_t copy_bytes() const { return (6 * fstride_ + psi_len_) * sizeof(S); }
+    FieldCopy copy_at(void* p) const {
+        S* const f = static_cast<S*>(p);
+        return FieldCopy{f, psi_len_ ? f + 6 * fstride_ : nullptr};
+    }
     FieldCopy cur_{}, other_{};
     size_t fstride_ = 0, psi_off_[6] = {}, psi_len_ = 0;
     S* fld(int c) const { return cur_.f + size_t(c) * fstride_ + xoff_; }
@@ -830,8 +947,6 @@ private:
         for (int c = 0; c < 6; ++c) *d[c] = f.f + size_t(c) * fstride_ + xoff_;
         for (int q = 0; q < 6; ++q) a.psiH[q] = f.psi ? f.psi + psi_off_[q] : nullptr;
     }
-    FieldCopy alloc_copy(bool zero);
-    void free_copy(FieldCopy& f);
     // One launch per step (fused.cuh): possible for this solve, its tiles, the tensor maps of the
     // copies ([copy read: 0 cur_ at the run's start, 1 other_][E, H]).
     bool fusable_ = false;
@@ -839,8 +954,14 @@ private:
     CUtensorMap maps_[2][2];
     const S* mapped_[2] = {};
     void setup_fused();
-    bool begin_fused();
+    void* new_copy();
+    void begin_fused(void* copy);
     void end_fused(uint64_t steps_run);
+    // steps that pay for a new second copy, of which the last kFusedLead are under way when it is
+    // asked for; steps taken without one
+    static constexpr uint64_t kFusedLead = 16;
+    uint64_t fused_pay_ = 0, fused_lead_ = kFusedLead, swept_ = 0;
+    IdleCopies::User copies_;
     void step_fused(const ESrc& src, int from);
     void pec_faces();  // PECBoundary after the E sweep: the faces of the planes this grid owns
     int timing_ = FDTD_TIMING_OFF;
@@ -1008,9 +1129,14 @@ Solver<S, T>::Solver(const fdtd_setup_v1& s, int dev, const ShardSpec* shard, bo
             psi_len_ += round_up(sz[q], 128 / sizeof(S));
         }
     }
-    cur_ = alloc_copy(true);
+    {
+        void* p = nullptr;
+        dev_alloc(&p, copy_bytes());
+        cur_ = copy_at(p);
+        ck(cudaMemsetAsync(p, 0, copy_bytes(), st_), "cudaMemsetAsync");
+    }
     point_args_at(a, cur_);
-    dev_bytes += (6 * fstride_ + psi_len_) * sizeof(S);
+    dev_bytes += copy_bytes();
 
     // bH must be uniform and aE = aH = 1 (sigma = 0, mu_r = 1).
     double bH = s.bH_uniform;
@@ -1342,43 +1468,27 @@ void Solver<S, T>::setup_fused() {
     // FDTD_B200_FUSED = 0 / 1: never / wherever possible.
     const double cells = double(NxT_) * NyT_ * NzT_;
     bool take = 5 * nv >= 4 * F::kMaxU * f.gx && cells >= (np_ == 0 ? 1e6 : sizeof(T) == 8 ? 8e6 : 2.5e7);
-    if (const char* e = std::getenv("FDTD_B200_FUSED")) take = std::string(e) != "0";
+    // A handle whose runs find no idle copy takes a new one when enough of its steps have gone without: the
+    // pool maps 6 - 9 ms per GB (1 ms and more for a small one), a fused step saves 3 us and more per
+    // million cells.  It asks for it after kFusedLead steps of a run, which the GPU takes about as
+    // long for: 536^3 FP64, first run of 10 and of 100 steps, two sweeps / copy mapped before the first
+    // step / so: 42.5 / 112 / 41 and 424 / 380 / 343 ms.
+    fused_pay_ = kFusedLead + uint64_t(350e6 / cells);
+    if (const char* e = std::getenv("FDTD_B200_FUSED")) {
+        take = std::string(e) != "0";
+        fused_pay_ = fused_lead_ = 0;
+    }
     // psi is addressed with 32-bit offsets
     const size_t xs = size_t(NzT_) * NyT_ * XSlab(NxT_, np_, W).len, ys = size_t(NzT_) * 2 * np_ * NxP_,
                  zs = size_t(2 * np_) * NyT_ * NxP_;
     fusable_ = take && a_.bidx != nullptr && std::max({xs, ys, zs, plane_}) < (size_t(1) << 31) && f.gy <= 65535 &&
                (NzT_ + f.kc - 1) / f.kc <= 65535;
     if (!fusable_) return;
+    copies_.join(device);
     fused_planes = uint64_t(f.kc);
     for (bool sh : {false, true})
         ck(cudaFuncSetAttribute(fused_kernel<T>(sh), cudaFuncAttributeMaxDynamicSharedMemorySize, int(F::bytes())),
            "cudaFuncSetAttribute");
-}
-
-template <typename S, typename T>
-typename Solver<S, T>::FieldCopy Solver<S, T>::alloc_copy(bool zero) {
-    FieldCopy f;
-    dev_alloc(reinterpret_cast<void**>(&f.f), 6 * fstride_ * sizeof(S));
-    if (psi_len_) {
-        try {
-            dev_alloc(reinterpret_cast<void**>(&f.psi), psi_len_ * sizeof(S));
-        } catch (...) {
-            dev_free(f.f);
-            throw;
-        }
-    }
-    if (zero) {
-        ck(cudaMemsetAsync(f.f, 0, 6 * fstride_ * sizeof(S), st_), "cudaMemsetAsync");
-        if (f.psi) ck(cudaMemsetAsync(f.psi, 0, psi_len_ * sizeof(S), st_), "cudaMemsetAsync");
-    }
-    return f;
-}
-
-template <typename S, typename T>
-void Solver<S, T>::free_copy(FieldCopy& f) {
-    if (f.f) dev_free(f.f);
-    if (f.psi) dev_free(f.psi);
-    f = FieldCopy{};
 }
 
 // cuTensorMapEncodeTiled from the driver the runtime has loaded (the library is not linked to it).
@@ -1399,14 +1509,11 @@ EncodeTiled encode_tiled() {
     return fn;
 }
 
-// The second copy of the fields for the steps of one run() call, from the stream-ordered pool (it
-// goes back at the call's end, so that between calls a solve holds what it held without it).
-// false: the run takes the two sweeps, in place -- no row-indexed material, or a device so full
-// that the copy would leave less than its own size free for other handles.
+// A second copy of the fields from the pool.  null: a device so full that the copy would leave less
+// than its own size free for others.
 template <typename S, typename T>
-bool Solver<S, T>::begin_fused() {
-    if (!fusable_ || path_ != 1 || timing_ == FDTD_TIMING_KERNELS || !encode_tiled()) return false;
-    const size_t bytes = (6 * fstride_ + psi_len_) * sizeof(S);
+void* Solver<S, T>::new_copy() {
+    const size_t bytes = copy_bytes();
     if (bytes > (size_t(256) << 20)) {
         size_t free_b = 0, total = 0;
         ck(cudaMemGetInfo(&free_b, &total), "cudaMemGetInfo");
@@ -1415,15 +1522,22 @@ bool Solver<S, T>::begin_fused() {
         uint64_t held = 0, used = 0;  // what the pool keeps for reuse is free too
         ck(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held), "cudaMemPoolGetAttribute");
         ck(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used), "cudaMemPoolGetAttribute");
-        if (free_b + (held - std::min(held, used)) < 2 * bytes) return false;
+        if (free_b + (held - std::min(held, used)) < 2 * bytes) return nullptr;
     }
-    try {
-        other_ = alloc_copy(false);
-    } catch (const Failure& f) {
-        if (f.code != FDTD_ERR_OOM) throw;
+    void* p = nullptr;
+    const cudaError_t e = cudaMallocAsync(&p, bytes, st_);
+    if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
-        return false;
+        return nullptr;
     }
+    ck(e, "cudaMallocAsync");
+    return p;
+}
+
+// The run's steps from here on are fused, from the current copy to `copy` and back.
+template <typename S, typename T>
+void Solver<S, T>::begin_fused(void* copy) {
+    other_ = copy_at(copy);
     using F = FusedShape<T>;
     const FieldCopy* const cp[2] = {&cur_, &other_};
     for (int b = 0; b < 2; ++b) {
@@ -1439,25 +1553,26 @@ bool Solver<S, T>::begin_fused() {
                                               one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                                               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
             if (r != CUDA_SUCCESS) {
-                free_copy(other_);
+                end_fused(0);
                 mapped_[0] = mapped_[1] = nullptr;
                 throw Failure(FDTD_ERR_CUDA, "cuTensorMapEncodeTiled failed");
             }
         }
         mapped_[b] = cp[b]->f;
     }
-    return true;
 }
 
-// The copy that holds the fields after `n` of the run's steps stays, the other goes back.
+// The copy that holds the fields after `n` of the run's steps stays, the other goes to the idle ones.
 template <typename S, typename T>
 void Solver<S, T>::end_fused(uint64_t n) {
+    cudaStreamSynchronize(st_);  // (a run that ends with an exception may not have waited)
     if (n & 1) {
         std::swap(cur_, other_);
         std::swap(mapped_[0], mapped_[1]);
         std::swap(maps_[0], maps_[1]);
     }
-    free_copy(other_);
+    IdleCopies::of(device).put(other_.f, copy_bytes());
+    other_ = FieldCopy{};
     point_args_at(a_, cur_);
 }
 
@@ -1543,8 +1658,7 @@ Solver<S, T>::~Solver() {
         if (trec_ev_[q]) cudaEventDestroy(trec_ev_[q]);
     for (auto& e : ev_) if (e) cudaEventDestroy(e);
     for (void* p : ptrs_) dev_free(p);
-    free_copy(cur_);
-    free_copy(other_);
+    if (cur_.f) dev_free(cur_.f);
     if (d_stage_) dev_free(d_stage_);
     if (d_series_) dev_free(d_series_);
     if (st_) cudaStreamDestroy(st_);
@@ -1793,14 +1907,26 @@ void Solver<S, T>::run(uint64_t n) {
     src_static(src);
     bool probe_due = false;
     const bool per_kernel = timing_ == FDTD_TIMING_KERNELS;
-    const bool fused = n > 0 && begin_fused();
-    struct Other {  // the workspace goes back whichever way the run ends
-        Solver* s;
+    struct Other {  // the second copy is given back whichever way the run ends
+        Solver* s = nullptr;
         uint64_t n = 0;
         ~Other() { if (s) s->end_fused(n); }
-    } other{fused ? this : nullptr};
+    } other;
+    // the first fused step, and the step before which a new second copy is asked for (past the end: none)
+    uint64_t f0 = last, ask = last + 1;
+    auto fuse_from = [&](uint64_t s, void* copy) {
+        if (!copy) return;
+        begin_fused(copy);
+        other.s = this;
+        f0 = s;
+    };
+    if (n > 0 && fusable_ && path_ == 1 && !per_kernel && encode_tiled()) {
+        fuse_from(n0, IdleCopies::of(device).take(copy_bytes()));
+        if (!other.s && swept_ + n >= fused_pay_) ask = n0 + std::min(n, fused_lead_);
+    }
     if (timing_ == FDTD_TIMING_RUN) ck(cudaEventRecord(ev_[0], st_), "cudaEventRecord");
     for (uint64_t s = n0; s < last; ++s) {
+        if (s == ask) fuse_from(s, new_copy());
         src_step(src, s);
         if (per_kernel) ck(cudaEventRecord(ev_[0], st_), "cudaEventRecord");
         if (path_ == 2) {
@@ -1813,10 +1939,11 @@ void Solver<S, T>::run(uint64_t n) {
             slabs<<<gridS_, blk, 0, st_>>>(a_, src, geom_, plan_, d_ctr_, d_status_);
             if (per_kernel) ck(cudaEventRecord(ev_[1], st_), "cudaEventRecord");
             launches += 1;
-        } else if (fused) {
-            step_fused(src, int((s - n0) & 1));
-            other.n = s + 1 - n0;
+        } else if (s >= f0) {
+            step_fused(src, int((s - f0) & 1));
+            other.n = s + 1 - f0;
         } else {
+            ++swept_;
             const size_t hmem = hpipe_ ? HPipe<S>::bytes() : 0;
             if (probe_due)
                 h_probe_kernel()<<<dim3(gridH_.x, gridH_.y, gridH_.z + 1), blk, hmem, st_>>>(a_, kchunkH_, geom_, src.step,
@@ -1835,7 +1962,7 @@ void Solver<S, T>::run(uint64_t n) {
             // along with the next step's H sweep instead of taking a launch of their own (us per step:
             // 48^3 21.7 -> 18, 80^3 25.2 -> 22, 157x121x93 46.5 -> 44.6, 173x131x97 FP64 122.8 -> 122;
             // above 2.5 M cells the launch is under 4 % of a step and is not seen)
-            probe_due = path_ == 1 && !fused && !per_kernel && probes_E_ && s + 1 < last && nflat_ <= 2500000;
+            probe_due = path_ == 1 && s < f0 && !per_kernel && probes_E_ && s + 1 < last && s + 1 != ask && nflat_ <= 2500000;
             if (!probe_due) launch_probes(s);
             if (s % save_every_ == 0) series_count_ = s / save_every_ + 1;
         }
@@ -1860,9 +1987,11 @@ void Solver<S, T>::run(uint64_t n) {
     }
     if (timing_ == FDTD_TIMING_RUN) ck(cudaEventRecord(ev_[3], st_), "cudaEventRecord");
     ck(cudaGetLastError(), "step kernels");
+    void* const next = ask == last ? new_copy() : nullptr;  // a short run: the copy is for the next one
     unsigned status = 0;
     ck(cudaMemcpyAsync(&status, d_status_, sizeof(unsigned), cudaMemcpyDeviceToHost, st_), "status");
     ck(cudaStreamSynchronize(st_), "run");
+    if (next) IdleCopies::of(device).put(next, copy_bytes());
     if (timing_ == FDTD_TIMING_RUN) {
         float ms = 0;
         ck(cudaEventElapsedTime(&ms, ev_[0], ev_[3]), "cudaEventElapsedTime");
@@ -1875,7 +2004,7 @@ void Solver<S, T>::run(uint64_t n) {
         MonitorState ms{};
         ck(cudaMemcpy(&ms, d_ms_, sizeof(ms), cudaMemcpyDeviceToHost), "monitor state");
         steps = ms.step + 1;
-        other.n = steps - n0;  // the launches after the failed monitor step did nothing
+        other.n = steps > f0 ? steps - f0 : 0;  // the launches after the failed monitor step did nothing
         series_count_ = std::min<uint64_t>(series_count_, (steps + save_every_ - 1) / save_every_);
         if (writer_) write_point_samples();
         throw Failure(FDTD_ERR_UNSTABLE, "stability monitor stopped the solve at step " + std::to_string(ms.step));

@@ -259,7 +259,8 @@ int fdtd_get_probe_series(fdtd_handle *h, double *out, uint64_t max_samples, uin
 /* DFT of probe p: X(f_m) = sum_n v(t_{n+1}) exp(-i 2 pi f_m t_{n+1}) dt, FP64. */
 int fdtd_get_dft(fdtd_handle *h, uint32_t probe, double *re, double *im);
 int fdtd_get_diagnostics(fdtd_handle *h, fdtd_diagnostics_v1 *out);
-/* Device memory held by the handle, bytes. */
+/* Device memory held by the handle, bytes.  Without the second copy of the fields (as much again as E,
+ * H and psi_H) that a large FP32 or FP64 solve's fdtd_run may use; it is shared by the handles of a device. */
 int fdtd_device_bytes(const fdtd_handle *h, uint64_t *bytes);
 /* Number of CUDA kernel launches issued by the handle since creation. */
 int fdtd_kernel_launches(const fdtd_handle *h, uint64_t *n);
@@ -274,7 +275,7 @@ int fdtd_set_timing(fdtd_handle *h, int mode);
 int fdtd_get_timing(fdtd_handle *h, fdtd_timing_v1 *out);
 /* Kernel path, before the first step only: 1 = the default (separate H and E sweeps or, for
  * FP32 and FP64 solves of a size that gains from it, one launch per step that reads the fields
- * from one copy and writes another; the second copy is held during fdtd_run only), 2 = one
+ * from one copy and writes another), 2 = one
  * persistent launch that runs the H and E sweeps slab by slab in dependency order (its
  * device waits are bounded; an expired wait makes fdtd_run return FDTD_ERR_TIMEOUT).  Both
  * paths give bit-identical results.  0 is reserved and refused with FDTD_ERR_UNSUPPORTED. */
