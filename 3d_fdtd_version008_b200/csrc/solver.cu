@@ -1457,17 +1457,28 @@ void Solver<S, T>::setup_fused() {
     }
     if (const char* e = std::getenv("FDTD_B200_FUSED_KCHUNK")) f.kc = std::clamp(std::atoi(e), 1, std::min(NzT_, int(F::kMaxKc)));
     // Which solves: a tile row takes a warp whatever it owns, so a row's vectors must fill most of
-    // its tiles (four fifths of 30 each); and a CPML slab costs the fused step more (its psi is
-    // loaded within a warp's plane, and one x-slab vector slows its whole row segment), so that
-    // the grid must be large enough for the saved HBM bytes to outweigh it.  Two sweeps -> fused, us
-    // per step, cubes with 10 - 12 CPML cells and gain unless noted: FP32 320^3 544 -> 511, 400^3
-    // 945 -> 916, 300x200x500 without gain 521 -> 486, 536^3 2162 -> 1880; but 200^3 175 -> 187,
-    // 236^3 257 -> 268, and where tiles are less full 280^3 (0.78) 353 -> 401.  FP64 200^3 283 -> 280,
-    // 236^3 437 -> 400, 280^3 663 -> 602, 400^3 1770 -> 1540, 536^3 4257 -> 3360; but 150^3 161 -> 169,
-    // 201x201x69 130 -> 156.  Without CPML (metal box 157x121x93) FP64 74 -> 59.
+    // its tiles; and a CPML slab costs the fused step more (its psi is loaded within a warp's plane,
+    // and one x-slab vector slows its whole row segment), so that the grid must be large enough for
+    // the saved HBM bytes to outweigh it.  A sheet makes the rows it touches take the general body
+    // (one normal to x, in every plane), which costs the fused step more too: with sheets the tiles
+    // must be fuller.  Two sweeps -> fused, us per step on the device, cubes with 10 - 12 CPML cells and
+    // gain unless noted (in brackets how full the tiles are):
+    //   FP32 300^3 (0.83) 484 -> 472, 320^3 542 -> 524, 400^3 (0.83) 923 -> 951, 420^3 1172 -> 1059, 500^3 (0.83)
+    //   1753 -> 1689, 536^3 2162 -> 1968; but 200^3 175 -> 187, 236^3 257 -> 268, 280^3 (0.78) 353 -> 401;
+    //   FP64 216^3 360 -> 330, 236^3 432 -> 411, 320^3 957 -> 901, 480^3 3159 -> 2492, 536^3 4257 -> 3435; but
+    //   196^3 270 -> 293, 208^3 294 -> 315;
+    //   a sheet normal to z, no gain: FP32 300^3 477 -> 490, 332^3 (0.92) 598 -> 602, 400^3 905 -> 1040, 440^3
+    //   (0.92) 1254 -> 1205; FP64 216^3 (0.90) 327 -> 352, 226^3 (0.94) 409 -> 371, 256^3 (0.85) 517 -> 558, 480^3
+    //   3069 -> 2689;
+    //   no CPML: FP32 100^3 38 -> 30, 200x100x100 (0.83) 45 -> 45, 216^3 169 -> 144, FP64 100^3 45 -> 43, 157x121x93
+    //   75 -> 58; a sheet normal to x too: FP32 216^3 (0.90) 191 -> 255, 232^3 (0.97) 288 -> 277, FP64 112^3
+    //   (0.93) 58 -> 60, 116x110x120 (0.97) 79 -> 66.
     // FDTD_B200_FUSED = 0 / 1: never / wherever possible.
-    const double cells = double(NxT_) * NyT_ * NzT_;
-    bool take = 5 * nv >= 4 * F::kMaxU * f.gx && cells >= (np_ == 0 ? 1e6 : sizeof(T) == 8 ? 8e6 : 2.5e7);
+    const double cells = double(NxT_) * NyT_ * NzT_, fill = double(nv) / (F::kMaxU * f.gx);
+    bool xsheet = false;
+    for (const auto& w : sheets_) xsheet |= w.axis == 0;
+    const double full = np_ != 0 && !sheets_.empty() ? 0.92 : xsheet ? 0.96 : 0.8;
+    bool take = fill >= full && cells >= (np_ == 0 ? 1e6 : sizeof(T) == 8 ? 1e7 : 2.5e7);
     // A handle whose runs find no idle copy takes a new one when enough of its steps have gone without: the
     // pool maps 6 - 9 ms per GB (1 ms and more for a small one), a fused step saves 3 us and more per
     // million cells.  It asks for it after kFusedLead steps of a run, which the GPU takes about as
