@@ -557,6 +557,7 @@ double field_scale_of(const fdtd_setup_v1& s, bool fp16) {
 struct ShardSpec {
     int kz0 = 0, NzG = 0, own0 = 0, own1 = 0;
     double psi_dx = 0;  // 16-bit storage: the whole solve's smallest cell edge (0: this grid's)
+    int sharing = 1;    // shards of the solve on this shard's device
 };
 
 // The second copies of the fields that fused steps write to (Solver::run), of one device: a run takes
@@ -1410,8 +1411,13 @@ Solver<S, T>::Solver(const fdtd_setup_v1& s, int dev, const ShardSpec* shard, bo
     const int gxH = g.gxi + (g.ne ? 1 : 0), gxE = gxi_E<S>(g) + (g.ne ? 1 : 0);
     const int gyE = std::max((NyT_ + rows_blk - 1) / rows_blk, g.ne ? (NyT_ + g.er - 1) / g.er : 0);
     // launch shapes: z-chunks by the rule of sweep_chunk
-    kchunkH_ = sweep_chunk(double(gxH) * ((NyT_ - 1 + rows_blk - 1) / rows_blk) * (NzT_ - 1));
-    kchunkE_ = sweep_chunk(double(gxE) * ((NyT_ + rows_blk - 1) / rows_blk) * NzT_);
+    // Shards that share a device: their sweeps overlap, so all their blocks count, and the last
+    // blocks of a launch seldom run alone (1.5).  us per step as 4 shards, chunks by each shard's own
+    // blocks -> so: 280^3 FP32 382 -> 351, FP64 741 -> 704, BF16 288 -> 251, 173x131x97 FP32 83 -> 75, 536^3 BF16
+    // 1440 -> 1396.
+    const double share = shard_.sharing > 1 ? 1.5 * shard_.sharing : 1.0;
+    kchunkH_ = sweep_chunk(share * gxH * ((NyT_ - 1 + rows_blk - 1) / rows_blk) * (NzT_ - 1));
+    kchunkE_ = sweep_chunk(share * gxE * ((NyT_ + rows_blk - 1) / rows_blk) * NzT_);
     if (const char* e = std::getenv("FDTD_B200_KCHUNK")) kchunkH_ = kchunkE_ = std::max(1, std::atoi(e));
     if (gyE > 65535) throw Failure(FDTD_ERR_INVALID, "grid too large for the sweep launch shape (NyT)");
     gridH_ = dim3(gxH, gyE, std::max(1, (a.kH1 + kchunkH_ - 1) / kchunkH_));
@@ -3149,7 +3155,8 @@ Sharded<S, T>::Sharded(const fdtd_setup_v1& s, int n, const int* devices) {
         }
         v.n_probes = uint32_t(sl->probes.size());
         v.probes = sl->probes.data();
-        ShardSpec spec{lo, int(NzT_), z0 - lo, z1 - lo, psi_dx};
+        ShardSpec spec{lo, int(NzT_), z0 - lo, z1 - lo, psi_dx, 0};
+        for (int q = 0; q < n; ++q) spec.sharing += (devices ? devices[q] : 0) == (devices ? devices[r] : 0);
         part_.push_back(std::make_unique<Solver<S, T>>(v, devices ? devices[r] : 0, &spec));
         slice_.push_back(std::move(sl));
     }
