@@ -14,6 +14,7 @@
 #include "kernels.cuh"
 
 #include <cuda_runtime.h>
+#include <omp.h>
 
 #include <algorithm>
 #include <array>
@@ -1694,7 +1695,7 @@ double* Solver<S, T>::staging() {
 // first large copy on the device and kept for the life of the process, so that creating and
 // destroying a solve neither pins nor unpins host memory.  A copy holds them (mu) throughout.
 struct PinnedChunks {
-    std::mutex mu;
+    std::mutex make, mu;
     void* buf[2] = {nullptr, nullptr};
     cudaEvent_t ev[2] = {nullptr, nullptr};
 };
@@ -1709,7 +1710,7 @@ PinnedChunks& pinned_chunks(int dev, size_t bytes) {
         if (!q) q = new PinnedChunks;
         p = q;
     }
-    std::lock_guard<std::mutex> l(p->mu);
+    std::lock_guard<std::mutex> l(p->make);
     for (int b = 0; b < 2; ++b) {
         if (!p->buf[b]) ck(cudaHostAlloc(&p->buf[b], bytes, cudaHostAllocDefault), "cudaHostAlloc");
         if (!p->ev[b]) ck(cudaEventCreateWithFlags(&p->ev[b], cudaEventDisableTiming), "cudaEventCreate");
@@ -1717,25 +1718,35 @@ PinnedChunks& pinned_chunks(int dev, size_t bytes) {
     return *p;
 }
 
-// memcpy split over the host threads (the pageable side of a chunk copy).  The destination is cut
+// memcpy split over `nt` host threads (the pageable side of a chunk copy).  The destination is cut
 // at multiples of `piece`: 2 MB pieces are whole huge pages, so that no two threads wait for the
-// same page of fresh memory.
-static void par_copy(void* dst, const void* src, size_t bytes, size_t piece = size_t(2) << 20) {
+// same page of fresh memory.  A destination that starts within a piece has a part of one at either
+// end: then the pieces are handed out as threads come free, so that no thread is left with two
+// (two threads reading 65 MB each into fresh memory 5.8 -> 5.1 ms); aligned ones (the pinned chunks)
+// go out in order, as a source read in order is 8 % faster.
+static void par_copy(void* dst, const void* src, size_t bytes, size_t piece = size_t(2) << 20,
+                     int nt = omp_get_max_threads()) {
     const size_t lead = (piece - reinterpret_cast<uintptr_t>(dst) % piece) % piece;
     const long long n = 1 + (long long)((bytes - std::min(lead, bytes) + piece - 1) / piece);
-#pragma omp parallel for schedule(static)
-    for (long long q = 0; q < n; ++q) {
+    auto copy = [=](long long q) {
         const size_t o = q == 0 ? 0 : lead + size_t(q - 1) * piece;
         const size_t e = std::min(bytes, lead + size_t(q) * piece);
         if (o < e) std::memcpy(static_cast<char*>(dst) + o, static_cast<const char*>(src) + o, e - o);
+    };
+    if (lead != 0) {
+#pragma omp parallel for schedule(dynamic) num_threads(nt)
+        for (long long q = 0; q < n; ++q) copy(q);
+    } else {
+#pragma omp parallel for schedule(static) num_threads(nt)
+        for (long long q = 1; q < n; ++q) copy(q);
     }
 }
-// First write to every page of a host array that is about to be overwritten, by all host threads.
-static void par_touch(void* dst, size_t bytes) {
+// First write to every page of a host array that is about to be overwritten, by nt host threads.
+static void par_touch(void* dst, size_t bytes, int nt) {
     const size_t piece = size_t(2) << 20;
     const size_t lead = (piece - reinterpret_cast<uintptr_t>(dst) % piece) % piece;
     const long long n = 1 + (long long)((bytes - std::min(lead, bytes) + piece - 1) / piece);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) num_threads(nt)
     for (long long q = 0; q < n; ++q) {
         const size_t e = std::min(bytes, lead + size_t(q) * piece);
         for (size_t o = q == 0 ? 0 : lead + size_t(q - 1) * piece; o < e; o += 4096)
@@ -1766,23 +1777,31 @@ void Solver<S, T>::h2d(const double* h, double* d, size_t n) {
 
 // The caller's array is usually fresh memory, whose pages are taken at the first write: one thread
 // (a plain cudaMemcpy) gets 5 GB/s.  From 1 MB on the copy therefore goes through a pinned chunk; an
-// array that fits one takes its pages with all host threads while the transfer runs.  Reads that
-// a program makes after a run: eight 22 MB arrays 38 -> 8 ms, six 14 MB ones 20 -> 3.7 ms.
+// array that fits one takes its pages with several host threads while the transfer runs.  Reads that
+// a program makes after a run: eight 22 MB arrays 38 -> 8 ms, six 14 MB ones 20 -> 3.7 ms.  Eight threads:
+// 16 are no faster, and their idle spinning slowed a second reading thread down.  A plain copy is
+// left to an array that is pinned (the DMA's own target: 22 MB 0.64 -> 0.42 ms) and to a reader that
+// finds the chunk taken by another thread (two threads, 14 MB each: plain 2.0 ms, waiting for the
+// chunk 3.0, so 1.0).
 template <typename S, typename T>
 void Solver<S, T>::d2h(const double* d, double* h, size_t n) {
-    if (n * sizeof(double) <= (size_t(1) << 20)) {
-        ck(cudaMemcpyAsync(h, d, n * sizeof(double), cudaMemcpyDeviceToHost, st_), "D2H");
-        ck(cudaStreamSynchronize(st_), "D2H");
-        return;
-    }
     if (n * sizeof(double) <= kPinBytes) {
         PinnedChunks& pc = pinned_chunks(device, kPinBytes);
-        std::lock_guard<std::mutex> l(pc.mu);
+        std::unique_lock<std::mutex> l(pc.mu, std::defer_lock);
+        cudaPointerAttributes at{};
+        if (n * sizeof(double) <= (size_t(1) << 20) || cudaPointerGetAttributes(&at, h) != cudaSuccess ||
+            at.type != cudaMemoryTypeUnregistered || !l.try_lock()) {
+            cudaGetLastError();  // (of the query)
+            ck(cudaMemcpyAsync(h, d, n * sizeof(double), cudaMemcpyDeviceToHost, st_), "D2H");
+            ck(cudaStreamSynchronize(st_), "D2H");
+            return;
+        }
         ck(cudaMemcpyAsync(pc.buf[0], d, n * sizeof(double), cudaMemcpyDeviceToHost, st_), "D2H");
         ck(cudaEventRecord(pc.ev[0], st_), "cudaEventRecord");
-        par_touch(h, n * sizeof(double));
+        const int nt = std::min(8, omp_get_max_threads());
+        par_touch(h, n * sizeof(double), nt);
         ck(cudaEventSynchronize(pc.ev[0]), "D2H");
-        par_copy(h, pc.buf[0], n * sizeof(double), size_t(1) << 18);
+        par_copy(h, pc.buf[0], n * sizeof(double), size_t(1) << 18, nt);
         return;
     }
     PinnedChunks& pc = pinned_chunks(device, kPinBytes);
