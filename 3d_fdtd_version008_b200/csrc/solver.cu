@@ -999,6 +999,23 @@ void keep_pool_memory(int dev) {
 // longer chunks save (536^3: 16 planes 1.107 ms, 34 planes 1.159 ms for the FP32 E sweep).
 int sweep_chunk(double bp) { return int(std::clamp(std::lround(std::sqrt(0.46 * bp / 296.0)), 1l, 16l)); }
 
+// The same without CPML, where the blocks (`tiles` columns of `planes` planes) cost alike and so tend to
+// leave in whole waves of 296: the time lies between whole and broken waves of chunks that take
+// their planes and 0.7 of a plane more, and a shorter tail of 0.3.  Fitted to 64^3 .. 200^3 in
+// FP32, FP64 and BF16 swept over c.  us per step, chunks of 8 planes and more / by the rule above / so:
+// 116x110x120 FP64 60 / 64 / 53, FP32 46 / 37 / 34, 140^3 FP64 105 / 114 / 105, 160^3 FP32 79 / 81 / 72, FP64
+// 138 / 142 / 137, BF16 74 / 67 / 65, 200^3 FP64 249 / 251 / 244.
+int sweep_chunk_even(int tiles, int planes) {
+    int best = 1;
+    double least = 1e300;
+    for (int c = 1; c <= 16; ++c) {
+        const double waves = double(tiles) * ((planes + c - 1) / c) / 296.0;
+        const double cost = 0.5 * (waves + std::ceil(waves)) * (c + 0.7) + 0.3 * c;
+        if (cost < least) { least = cost; best = c; }
+    }
+    return best;
+}
+
 // The setup's full-grid checks that need no device: the material index's range and the gain
 // cells' bounding box and placement.  A large solve runs them on a helper thread while it
 // allocates its device arrays (for a 536^3 first solve both take tens of milliseconds: growing
@@ -1417,8 +1434,14 @@ Solver<S, T>::Solver(const fdtd_setup_v1& s, int dev, const ShardSpec* shard, bo
     // blocks -> so: 280^3 FP32 382 -> 351, FP64 741 -> 704, BF16 288 -> 251, 173x131x97 FP32 83 -> 75, 536^3 BF16
     // 1440 -> 1396.
     const double share = shard_.sharing > 1 ? 1.5 * shard_.sharing : 1.0;
-    kchunkH_ = sweep_chunk(share * gxH * ((NyT_ - 1 + rows_blk - 1) / rows_blk) * (NzT_ - 1));
-    kchunkE_ = sweep_chunk(share * gxE * ((NyT_ + rows_blk - 1) / rows_blk) * NzT_);
+    const int tyH = (NyT_ - 1 + rows_blk - 1) / rows_blk, tyE = (NyT_ + rows_blk - 1) / rows_blk;
+    if (np_ > 0) {
+        kchunkH_ = sweep_chunk(share * gxH * tyH * (NzT_ - 1));
+        kchunkE_ = sweep_chunk(share * gxE * tyE * NzT_);
+    } else {
+        kchunkH_ = sweep_chunk_even(shard_.sharing * gxH * tyH, NzT_ - 1);
+        kchunkE_ = sweep_chunk_even(shard_.sharing * gxE * tyE, NzT_);
+    }
     if (const char* e = std::getenv("FDTD_B200_KCHUNK")) kchunkH_ = kchunkE_ = std::max(1, std::atoi(e));
     if (gyE > 65535) throw Failure(FDTD_ERR_INVALID, "grid too large for the sweep launch shape (NyT)");
     gridH_ = dim3(gxH, gyE, std::max(1, (a.kH1 + kchunkH_ - 1) / kchunkH_));
@@ -1477,15 +1500,16 @@ void Solver<S, T>::setup_fused() {
     //   a sheet normal to z, no gain: FP32 300^3 477 -> 490, 332^3 (0.92) 598 -> 602, 400^3 905 -> 1040, 440^3
     //   (0.92) 1254 -> 1205; FP64 216^3 (0.90) 327 -> 352, 226^3 (0.94) 409 -> 371, 256^3 (0.85) 517 -> 558, 480^3
     //   3069 -> 2689;
-    //   no CPML: FP32 100^3 38 -> 30, 200x100x100 (0.83) 45 -> 45, 216^3 169 -> 144, FP64 100^3 45 -> 43, 157x121x93
-    //   75 -> 58; a sheet normal to x too: FP32 216^3 (0.90) 191 -> 255, 232^3 (0.97) 288 -> 277, FP64 112^3
-    //   (0.93) 58 -> 60, 116x110x120 (0.97) 79 -> 66.
+    //   no CPML: FP32 104^3 30.2 -> 30.2, 120^3 34 -> 37, 200x100x100 42 -> 45, 208x140x120 69 -> 61, 180^3 (0.75) 110 ->
+    //   102, 216^3 163 -> 144, 280^3 (0.78) 359 -> 291; FP64 104^3 42 -> 44, 108^3 45 -> 43, 157x121x93 72 -> 59, 136^3
+    //   (0.76) 99 -> 90, 280^3 594 -> 464; a sheet normal to x too: FP32 216^3 (0.90) 194 -> 256, 232^3 (0.97) 288 ->
+    //   277, FP64 112^3 (0.93) 56 -> 61, 116x110x120 (0.97) 76 -> 67.
     // FDTD_B200_FUSED = 0 / 1: never / wherever possible.
     const double cells = double(NxT_) * NyT_ * NzT_, fill = double(nv) / (F::kMaxU * f.gx);
     bool xsheet = false;
     for (const auto& w : sheets_) xsheet |= w.axis == 0;
-    const double full = np_ != 0 && !sheets_.empty() ? 0.92 : xsheet ? 0.96 : 0.8;
-    bool take = fill >= full && cells >= (np_ == 0 ? 1e6 : sizeof(T) == 8 ? 1e7 : 2.5e7);
+    const double full = np_ != 0 ? (sheets_.empty() ? 0.8 : 0.92) : xsheet ? 0.96 : 0.75;
+    bool take = fill >= full && cells >= (np_ == 0 ? (sizeof(T) == 8 ? 1.25e6 : 3e6) : sizeof(T) == 8 ? 1e7 : 2.5e7);
     // A handle whose runs find no idle copy takes a new one when enough of its steps have gone without: the
     // pool maps 6 - 9 ms per GB (1 ms and more for a small one), a fused step saves 3 us and more per
     // million cells.  It asks for it after kFusedLead steps of a run, which the GPU takes about as

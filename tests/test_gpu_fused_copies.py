@@ -91,7 +91,7 @@ def test_copy_is_taken_when_steps_pay(pkg, monkeypatch):
     pay = 16 + int(350e6 / (n[0] * n[1] * n[2]))
     got, per_step = [], []
     for runs in ((10, pay - 11, 1, 10), (pay + 5, 10)):  # short runs that come to `pay` steps; one long run
-        sol = _solver(pkg, text, 2)
+        sol = _solver(pkg, text, 2, precision=1)
         assert sol.fused_planes > 0
         for k in runs:
             l0 = sol.kernel_launches
@@ -104,7 +104,25 @@ def test_copy_is_taken_when_steps_pay(pkg, monkeypatch):
     assert one < per_step[4] < one + 0.5 * (two - one) and per_step[5] == one
     monkeypatch.setenv("FDTD_B200_FUSED", "0")
     for runs, g in zip(((10, pay - 11, 1, 10), (pay + 5, 10)), got):
-        ref = _solver(pkg, text, 2)
+        ref = _solver(pkg, text, 2, precision=1)
         ref.run(sum(runs))
         assert all(np.array_equal(x, y) for x, y in zip(g, _state(ref)))
         ref.close()
+
+
+@pytest.mark.gpu
+def test_probes_ride_up_to_the_first_fused_step(pkg, monkeypatch):
+    """E-only probes ride with the next H sweep; the step before the first fused one has no such sweep."""
+    n = (116, 100, 110)
+    text = _params(n, 0, boundary=0).replace(", 2, 4\n", ", 2\n").replace("SAVE_EVERY = 2", "SAVE_EVERY = 1")
+    out = []
+    for fused in (None, "0"):
+        if fused:
+            monkeypatch.setenv("FDTD_B200_FUSED", fused)
+        sol = _solver(pkg, text, 4, precision=1)
+        assert sol.n_probes == 1 and (sol.fused_planes > 0) == (fused is None)
+        sol.run(320)
+        sol.run(3)
+        out.append(_state(sol) + [sol.dft(0)])
+        sol.close()
+    assert all(np.array_equal(a, b) for a, b in zip(*out))

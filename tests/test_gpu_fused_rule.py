@@ -6,8 +6,9 @@ from test_gpu_fused import DS, _params
 SHEET = {"x": (0, 2), "z": (4, 0)}  # direction, polarization
 CASES = [
     # (cells, npml, sheets, precision, one launch)
-    ((100, 100, 100), 0, "", 0, True), ((96, 100, 100), 0, "", 0, False), ((92, 120, 120), 0, "", 0, False),
-    ((100, 100, 100), 0, "z", 1, True), ((100, 100, 100), 0, "xz", 1, False), ((116, 100, 100), 0, "xz", 1, True),
+    ((180, 180, 92), 0, "", 0, False), ((180, 180, 94), 0, "", 0, True), ((176, 180, 100), 0, "", 0, False),
+    ((104, 110, 110), 0, "z", 1, True), ((104, 104, 104), 0, "z", 1, False), ((104, 110, 120), 0, "xz", 1, False),
+    ((116, 110, 110), 0, "xz", 1, True),
     ((216, 215, 216), 8, "", 1, True), ((208, 208, 208), 8, "", 1, False), ((216, 215, 216), 8, "z", 1, False),
     ((226, 226, 226), 8, "z", 1, True), ((230, 300, 360), 8, "", 0, False),
 ]
