@@ -5,8 +5,9 @@
 // slabs, the gain block (bounding box of the gain cells: region id, P ping-pong, Nu,
 // Ng), probe series / DFT accumulators and the stability-monitor state.  fdtd_run()
 // issues, per step, k_step_fused or k_update_H and k_update_E, the probe/DFT kernel and on monitor steps
-// the FP64 diagnostic reduction, on the handle's stream.  All device memory comes from
-// cudaMalloc at create time (staging for layout transposes on first use).
+// the FP64 diagnostic reduction, on the handle's stream.  A handle's device memory comes from the
+// stream-ordered pool at create time (staging for layout transposes on first use, the probe series as
+// it grows); fused steps use a second copy of the fields besides (IdleCopies).
 #include "../../include/fdtd_b200.h"
 #include "host/outputs.hpp"
 #include "host/waveform.hpp"
@@ -1127,8 +1128,7 @@ Solver<S, T>::Solver(const fdtd_setup_v1& s, int dev, const ShardSpec* shard, bo
     a.kE0 = std::max(shard_.own0, 1 - shard_.kz0);
     a.kE1 = shard_.own1;
     // A whole single solve in FP32 or FP64 may step with one fused launch: it needs the row-indexed
-    // material (known below) and the pool (its second copy of the fields is a workspace of each
-    // run).  The switches that shape the two sweeps select the two sweeps.
+    // material (known below) and the pool (its second copy of the fields comes from there).  The switches that shape the two sweeps select the two sweeps.
     fusable_ = std::is_same_v<S, T> && !shard && !pooled && pooled_;
     for (const char* v : {"FDTD_B200_LANES", "FDTD_B200_KCHUNK", "FDTD_B200_H_PIPE", "FDTD_B200_E_PIPE"})
         if (std::getenv(v)) fusable_ = false;
@@ -2019,9 +2019,11 @@ void Solver<S, T>::run(uint64_t n) {
         if (per_kernel) ck(cudaEventRecord(ev_[2], st_), "cudaEventRecord");
         if (nprobes_) {
             // E does not change until the next E sweep: on a small grid, probes that read only E ride
-            // along with the next step's H sweep instead of taking a launch of their own (us per step:
-            // 48^3 21.7 -> 18, 80^3 25.2 -> 22, 157x121x93 46.5 -> 44.6, 173x131x97 FP64 122.8 -> 122;
-            // above 2.5 M cells the launch is under 4 % of a step and is not seen)
+            // along with the next step's H sweep instead of taking a launch of their own.  us per step,
+            // own launch -> ride, FP32 / FP64: 48^3 19.5 -> 15.4 / 19.5 -> 15.4, 80^3 27.0 -> 24.7 / 31.8 -> 29.3, 128^3
+            // 52.4 -> 52.2 / 93.4 -> 92.8, 173x131x97 (2.4 M padded cells) 63.3 -> 63.4 / 109.7 -> 108.1; above that the
+            // sweep's second form costs what the launch did or more: 201x201x69 77.9 -> 79.2 / 129.4 -> 127.4, 200^3
+            // 176.2 -> 175.0 / 281.2 -> 283.4, 280^3 352 -> 356 / 648 -> 659.
             probe_due = path_ == 1 && s < f0 && !per_kernel && probes_E_ && s + 1 < last && s + 1 != ask && nflat_ <= 2500000;
             if (!probe_due) launch_probes(s);
             if (s % save_every_ == 0) series_count_ = s / save_every_ + 1;
