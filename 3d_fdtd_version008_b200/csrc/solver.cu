@@ -1495,8 +1495,8 @@ void Solver<S, T>::setup_fused() {
     // gain unless noted (in brackets how full the tiles are):
     //   FP32 300^3 (0.83) 484 -> 472, 320^3 542 -> 524, 400^3 (0.83) 923 -> 951, 420^3 1172 -> 1059, 500^3 (0.83)
     //   1753 -> 1689, 536^3 2162 -> 1968; but 200^3 175 -> 187, 236^3 257 -> 268, 280^3 (0.78) 353 -> 401;
-    //   FP64 216^3 360 -> 330, 236^3 432 -> 411, 320^3 957 -> 901, 480^3 3159 -> 2492, 536^3 4257 -> 3435; but
-    //   196^3 270 -> 293, 208^3 294 -> 315;
+    //   FP64 158x263x221 (0.88) 320 -> 294, 216^3 360 -> 330, 236^3 432 -> 411, 320^3 957 -> 901, 480^3 3159 -> 2492, 536^3 4257 -> 3435; but
+    //   196^3 (0.82) 270 -> 293, 208^3 (0.87) 294 -> 315;
     //   a sheet normal to z, no gain: FP32 300^3 477 -> 490, 332^3 (0.92) 598 -> 602, 400^3 905 -> 1040, 440^3
     //   (0.92) 1254 -> 1205; FP64 216^3 (0.90) 327 -> 352, 226^3 (0.94) 409 -> 371, 256^3 (0.85) 517 -> 558, 480^3
     //   3069 -> 2689;
@@ -1509,7 +1509,8 @@ void Solver<S, T>::setup_fused() {
     bool xsheet = false;
     for (const auto& w : sheets_) xsheet |= w.axis == 0;
     const double full = np_ != 0 ? (sheets_.empty() ? 0.8 : 0.92) : xsheet ? 0.96 : 0.75;
-    bool take = fill >= full && cells >= (np_ == 0 ? (sizeof(T) == 8 ? 1.25e6 : 3e6) : sizeof(T) == 8 ? 1e7 : 2.5e7);
+    bool take = fill >= full && (np_ == 0 ? cells >= (sizeof(T) == 8 ? 1.25e6 : 3e6)
+                                          : sizeof(T) == 8 ? cells * fill >= 8e6 : cells >= 2.5e7);
     // A handle whose runs find no idle copy takes a new one when enough of its steps have gone without: the
     // pool maps 6 - 9 ms per GB (1 ms and more for a small one), a fused step saves 3 us and more per
     // million cells.  It asks for it after kFusedLead steps of a run, which the GPU takes about as
@@ -1802,8 +1803,9 @@ void Solver<S, T>::h2d(const double* h, double* d, size_t n) {
 // The caller's array is usually fresh memory, whose pages are taken at the first write: one thread
 // (a plain cudaMemcpy) gets 5 GB/s.  From 1 MB on the copy therefore goes through a pinned chunk; an
 // array that fits one takes its pages with several host threads while the transfer runs.  Reads that
-// a program makes after a run: eight 22 MB arrays 38 -> 8 ms, six 14 MB ones 20 -> 3.7 ms.  Eight threads:
-// 16 are no faster, and their idle spinning slowed a second reading thread down.  A plain copy is
+// a program makes after a run: eight 22 MB arrays 38 -> 8 ms, six 14 MB ones 20 -> 3.7 ms.  Twelve
+// threads: six 22 MB arrays take one reader 5.4 ms with 8, 4.9 with 12, 4.6 with 16, and two readers at
+// once 13, 13 and 16 - 20, as idle threads spin.  A plain copy is
 // left to an array that is pinned (the DMA's own target: 22 MB 0.64 -> 0.42 ms) and to a reader that
 // finds the chunk taken by another thread (two threads, 14 MB each: plain 2.0 ms, waiting for the
 // chunk 3.0, so 1.0).
@@ -1822,7 +1824,7 @@ void Solver<S, T>::d2h(const double* d, double* h, size_t n) {
         }
         ck(cudaMemcpyAsync(pc.buf[0], d, n * sizeof(double), cudaMemcpyDeviceToHost, st_), "D2H");
         ck(cudaEventRecord(pc.ev[0], st_), "cudaEventRecord");
-        const int nt = std::min(8, omp_get_max_threads());
+        const int nt = std::min(12, omp_get_max_threads());
         par_touch(h, n * sizeof(double), nt);
         ck(cudaEventSynchronize(pc.ev[0]), "D2H");
         par_copy(h, pc.buf[0], n * sizeof(double), size_t(1) << 18, nt);

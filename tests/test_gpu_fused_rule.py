@@ -9,7 +9,7 @@ CASES = [
     ((180, 180, 92), 0, "", 0, False), ((180, 180, 94), 0, "", 0, True), ((176, 180, 100), 0, "", 0, False),
     ((104, 110, 110), 0, "z", 1, True), ((104, 104, 104), 0, "z", 1, False), ((104, 110, 120), 0, "xz", 1, False),
     ((116, 110, 110), 0, "xz", 1, True),
-    ((216, 215, 216), 8, "", 1, True), ((208, 208, 208), 8, "", 1, False), ((216, 215, 216), 8, "z", 1, False),
+    ((216, 215, 216), 8, "", 1, True), ((208, 208, 208), 8, "", 1, False), ((158, 262, 222), 8, "", 1, True), ((216, 215, 216), 8, "z", 1, False),
     ((226, 226, 226), 8, "z", 1, True), ((230, 300, 360), 8, "", 0, False),
 ]
 
