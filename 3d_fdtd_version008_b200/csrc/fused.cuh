@@ -23,13 +23,12 @@
 //
 // What bounds it: 24 (FP32) bytes are read and 24 written per cell and step, so HBM is the floor; the
 // copies in flight (two blocks of 26 KB stages, two planes ahead) and the 16 warps' instruction
-// latencies keep it at 0.7 - 0.75 of the measured copy bandwidth in plain planes.  Hence everything
+// latencies keep it at 0.81 (FP64) and 0.73 (FP32) of the measured copy bandwidth on 536^3.  Hence everything
 // a plane waits for comes from shared memory (coefficients, material rows) or is asked for
 // one plane ahead (psi, row numbers: L2 prefetch), FP32 arithmetic runs on pairs of cells, and
 // the kernel has to fit 128 registers exactly: with the shared memory in use L1 holds next to
 // nothing, and a spilled value costs an L2 trip (a build with 100 spilled bytes ran 15 - 30 % slower).
-// Measured, 536^3 CPML + gain, one B200, us per step with probe and monitor: two sweeps -> fused
-// FP32 2217 -> 1880, FP64 4329 -> 3360 (sizes in between: Solver's rule).
+// Against the two sweeps it is measured, size by size, at Solver's rule (setup_fused in solver.cu).
 //
 // psi_H is needed by the blocks that recompute a neighbour's H too, so it also alternates
 // between two copies; psi_E, P (two slots already), Nu and Ng are touched by their owner alone.

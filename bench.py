@@ -10,7 +10,7 @@ steps (default 10).  The headline is the FP64 mode, the reference's own arithmet
 total cell-updates / device time of K bench steps, in Mcell-updates/s, measured with CUDA
 events on the library's stream(s) bracketed by barriers and synchronisation, max over ranks.
 FP32, BF16 and FP16 storage are measured in the same run (--forms) as blocks of the line, each
-with its roofline (per-kernel events of a whole solve) and its accuracy against the FP64 solve
+with its roofline (events around its kernels on a whole solve) and its accuracy against the FP64 solve
 after the same W + K runs from the same state.  The field state (3.7-7.4 GB) is far larger
 than L2 (126 MB), so no L2 flush is needed.
 
@@ -133,7 +133,8 @@ def algorithmic_bytes(setup, word: int, coef_word: int = 0, material_bytes: int 
     E(3) = 9 field words + the material (bE: 3 coefficient words per cell, or `material_bytes`
     per cell when the stepper holds it as a row index -- the small row table stays on chip);
     + 2 field words per active CPML psi (4 per axis, 2 per sweep) in that axis' slab; + gain
-    cells: read P^n, P^{n-1}, Nu, Ng and write P^{n+1}, Nu, Ng = 7 coefficient words."""
+    cells: read P^n, P^{n-1}, Nu, Ng and write P^{n+1}, Nu, Ng = 7 coefficient words.  fused_bytes:
+    the same for the one-launch step, which reads and writes E and H once (12 field words)."""
     cw = coef_word or word
     mat = material_bytes or 3 * cw
     NxT, NyT, NzT = setup.shape
@@ -143,7 +144,8 @@ def algorithmic_bytes(setup, word: int, coef_word: int = 0, material_bytes: int 
     gain = int((setup.array("tls_region_map") >= 0).sum()) if setup.view.n_tls_regions else 0
     h = 9 * word * cells + 2 * 2 * word * slab
     e = 9 * word * cells + mat * cells + 2 * 2 * word * slab + 7 * cw * gain
-    return {"cells": cells, "h_bytes": h, "e_bytes": e, "step_bytes": h + e,
+    one = h + e - 6 * word * cells
+    return {"fused_bytes": one, "fused_per_cell": one / cells, "cells": cells, "h_bytes": h, "e_bytes": e, "step_bytes": h + e,
             "per_cell": (h + e) / cells, "slab_cells": slab, "gain_cells": gain}
 
 
@@ -635,9 +637,8 @@ DTYPE = {"fp32": "f32", "fp64": "f64", "fp16": "f32 (fp16 storage)", "bf16": "f3
 def shards_for(args, form: str) -> int:
     """z shards of the solve on the GPU for a storage form: --shards, else the fastest measured
     on the 536^3 workload (one B200): FP64 and FP32 step fastest whole, with one launch per step
-    (45 and 80 Gcell-updates/s; 36.5 and 72.6 as 4 shards, which take two sweeps); BF16 and FP16
-    with 4 shards (101.8 / 104.6 against 97.5 / 100.8 whole, in an earlier build), whose sweeps'
-    tails overlap on their streams."""
+    (47 and 83 Gcell-updates/s; 36 and 72 as 4 shards, which take two sweeps); BF16 and FP16
+    with 4 shards, whose sweeps' tails overlap on their streams (BF16 1.40 against 1.45 ms a step whole)."""
     if args.shards:
         return args.shards
     return 1 if form in ("fp64", "fp32") else 4
@@ -823,11 +824,34 @@ def accuracy(sols: dict, ref) -> dict:
 
 
 def kernel_roofline(setup, form: str, S: int, K: int, local: int) -> dict:
-    """Per-kernel CUDA events (one synchronisation per step) on a whole solve of the workload:
-    the E sweep's algorithmic bytes per launch over its average launch time, against the
-    measured copy bandwidth of this pool's B200s."""
+    """The step's kernels on a whole solve of the workload: algorithmic bytes per launch over the
+    average launch time, against the measured copy bandwidth of this pool's B200s.  Two sweeps:
+    per-kernel CUDA events (one synchronisation per step), the E sweep named.  The one-launch
+    step: the events around runs of a solve without probes and monitor, which launch nothing else."""
     word = WORD[form]
     coef_word = 8 if form == "fp64" else 4
+    peak, peak_src = peaks()
+    view = PKG.SetupV1.from_buffer_copy(setup.view)
+    view.n_probes = view.monitor_interval = 0
+    sol = PKG.Solver(setup, device=local, precision=PREC[form], view=view if form in ("fp64", "fp32") else None)
+    if sol.fused_planes:
+        alg = algorithmic_bytes(setup, word, coef_word, 2 if sol.material_rows else 0)
+        for _ in range(2):
+            sol.run(max(40, S))  # the second copy of the fields is taken in the first
+        sol.set_timing(PKG.TIMING_RUN)
+        before = sol.kernel_launches
+        for _ in range(min(K, 5)):
+            sol.run(S)
+        tm = sol.timing()
+        assert sol.kernel_launches - before == tm["steps"]
+        sol.close()
+        ms = tm["run_ms"] / tm["steps"]
+        achieved = round(alg["fused_bytes"] / (ms * 1e-3) / 1e9, 1)
+        return {"roofline": {"bound": "hbm", "kernel": "k_step_fused", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                             "frac": round(achieved / peak, 4), "peak_source": peak_src, "traffic": None,
+                             "algorithmic_bytes_per_launch": alg["fused_bytes"], "avg_launch_ms": round(ms, 5)},
+                "hbm_gbs_step": achieved, "per_cell": round(alg["fused_per_cell"], 2)}
+    sol.close()
     sol = PKG.Solver(setup, device=local, precision=PREC[form])
     alg = algorithmic_bytes(setup, word, coef_word, 2 if sol.material_rows else 0)
     sol.run(S)
@@ -838,7 +862,6 @@ def kernel_roofline(setup, form: str, S: int, K: int, local: int) -> dict:
     sol.close()
     e_ms = tm["e_ms"] / tm["steps"]
     h_ms = tm["h_ms"] / tm["steps"]
-    peak, peak_src = peaks()
     achieved = alg["e_bytes"] / (e_ms * 1e-3) / 1e9
     traffic = None
     prof = ROOT / "profiles" / f"k_update_E_b512_{form}_traffic.json"
@@ -1000,8 +1023,10 @@ def main():
                                    ("replicas, one per GPU" if world > 1 else "single GPU")
                                    + (f", {shards_for(args, head)} z-shards of the solve overlapped on the GPU"
                                       if shards_for(args, head) > 1 else "")),
-                   "roofline_timing": "whole (unsharded) solve, per-kernel CUDA events on the library's stream",
-                   "kernel_path": "separate H and E sweeps",
+                   "roofline_timing": "whole (unsharded) solve, CUDA events on the library's stream around the named "
+                                      "kernel (k_step_fused: around runs that launch nothing else)",
+                   "kernel_path": ("one launch per step (k_step_fused)" if roof[head]["roofline"]["kernel"] == "k_step_fused"
+                                   and not shard_devs and shards_for(args, head) == 1 else "separate H and E sweeps"),
                    "l2": "state (%.1f GB of fields) larger than L2 (126 MB), no flush" % (cells * WORD[head] * 6 / 1e9),
                    "wall_ms_per_step": round(h["wall_ms"] / K, 4),
                    "accuracy_note": "each form against the FP64 solve after the same W + K runs of S steps "
