@@ -657,8 +657,13 @@ private:
         int now = 0;
         cudaGetDevice(&now);
         cudaSetDevice(dev_);
-        for (const Buf& b : out) cudaFreeAsync(b.p, cudaStreamPerThread);
-        cudaStreamSynchronize(cudaStreamPerThread);  // now any stream's allocation may have them
+        // on a stream that ends here: what a living stream has freed the pool gives to other streams
+        // only after a look at that stream (a later batch of packed jobs ran 3.5 % slower)
+        cudaStream_t st = nullptr;
+        if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) st = cudaStreamPerThread;
+        for (const Buf& b : out) cudaFreeAsync(b.p, st);
+        cudaStreamSynchronize(st);
+        if (st != cudaStreamPerThread) cudaStreamDestroy(st);
         cudaSetDevice(now);
     }
     static constexpr size_t kIdle = 4;
